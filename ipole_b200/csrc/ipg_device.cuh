@@ -591,6 +591,30 @@ __device__ __forceinline__ void hn_unpack(const HermN &n, double R[4][4], double
   S[3][0] = -n.s03; S[3][1] = -n.s13; S[3][2] = -n.s23; S[3][3] = 0.;
 }
 
+/* The transfer's linear algebra is written with its roundings spelled out
+ * (explicit fused and unfused operations): the walks exist as one lane per
+ * ray and as four lanes per ray, each sharing out the sums differently, and
+ * every form must give the same bits whatever the compiler would contract. */
+__device__ __forceinline__ double dot4_rn(double a0, double a1, double a2, double a3, double b0, double b1, double b2,
+                                          double b3)
+{
+  return __fma_rn(a3, b3, __fma_rn(a2, b2, __fma_rn(a0, b0, __dmul_rn(a1, b1))));
+}
+__device__ __forceinline__ double dot4_rn(const double a[4], const double b[4])
+{
+  return dot4_rn(a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3]);
+}
+/* the sum in the order of a butterfly over four lanes (never contracted) */
+__device__ __forceinline__ double sum4_rn(double p0, double p1, double p2, double p3)
+{
+  return __dadd_rn(__dadd_rn(p0, p1), __dadd_rn(p2, p3));
+}
+__device__ __forceinline__ float dot4f_rn(float a0, float a1, float a2, float a3, float b0, float b1, float b2,
+                                          float b3)
+{
+  return __fmaf_rn(a3, b3, __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1))));
+}
+
 /* out = base - dl (A M + M A^T), M Hermitian (push_polar, src/ipolarray.c:277-287) */
 __device__ __forceinline__ void hn_push(const HermN &base, const HermN &Mh, const double A[4][4], double dl, HermN *out)
 {
@@ -600,25 +624,29 @@ __device__ __forceinline__ void hn_push(const HermN &base, const HermN &Mh, cons
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      AR[i][j] = A[i][0] * R[0][j] + A[i][1] * R[1][j] + A[i][2] * R[2][j] + A[i][3] * R[3][j];
-      AS[i][j] = A[i][0] * S[0][j] + A[i][1] * S[1][j] + A[i][2] * S[2][j] + A[i][3] * S[3][j];
+      AR[i][j] = dot4_rn(A[i][0], A[i][1], A[i][2], A[i][3], R[0][j], R[1][j], R[2][j], R[3][j]);
+      AS[i][j] = dot4_rn(A[i][0], A[i][1], A[i][2], A[i][3], S[0][j], S[1][j], S[2][j], S[3][j]);
     }
-  out->r00 = base.r00 - dl * (AR[0][0] + AR[0][0]);
-  out->r01 = base.r01 - dl * (AR[0][1] + AR[1][0]);
-  out->r02 = base.r02 - dl * (AR[0][2] + AR[2][0]);
-  out->r03 = base.r03 - dl * (AR[0][3] + AR[3][0]);
-  out->r11 = base.r11 - dl * (AR[1][1] + AR[1][1]);
-  out->r12 = base.r12 - dl * (AR[1][2] + AR[2][1]);
-  out->r13 = base.r13 - dl * (AR[1][3] + AR[3][1]);
-  out->r22 = base.r22 - dl * (AR[2][2] + AR[2][2]);
-  out->r23 = base.r23 - dl * (AR[2][3] + AR[3][2]);
-  out->r33 = base.r33 - dl * (AR[3][3] + AR[3][3]);
-  out->s01 = base.s01 - dl * (AS[0][1] - AS[1][0]);
-  out->s02 = base.s02 - dl * (AS[0][2] - AS[2][0]);
-  out->s03 = base.s03 - dl * (AS[0][3] - AS[3][0]);
-  out->s12 = base.s12 - dl * (AS[1][2] - AS[2][1]);
-  out->s13 = base.s13 - dl * (AS[1][3] - AS[3][1]);
-  out->s23 = base.s23 - dl * (AS[2][3] - AS[3][2]);
+#define PR(b, i, j) __fma_rn(-dl, __dadd_rn(AR[i][j], AR[j][i]), b)
+#define PS(b, i, j) __fma_rn(-dl, __dsub_rn(AS[i][j], AS[j][i]), b)
+  out->r00 = PR(base.r00, 0, 0);
+  out->r01 = PR(base.r01, 0, 1);
+  out->r02 = PR(base.r02, 0, 2);
+  out->r03 = PR(base.r03, 0, 3);
+  out->r11 = PR(base.r11, 1, 1);
+  out->r12 = PR(base.r12, 1, 2);
+  out->r13 = PR(base.r13, 1, 3);
+  out->r22 = PR(base.r22, 2, 2);
+  out->r23 = PR(base.r23, 2, 3);
+  out->r33 = PR(base.r33, 3, 3);
+  out->s01 = PS(base.s01, 0, 1);
+  out->s02 = PS(base.s02, 0, 2);
+  out->s03 = PS(base.s03, 0, 3);
+  out->s12 = PS(base.s12, 1, 2);
+  out->s13 = PS(base.s13, 1, 3);
+  out->s23 = PS(base.s23, 2, 3);
+#undef PR
+#undef PS
 }
 
 /* Stokes parameters of N in a tetrad with covariant rows e1 = Ecov[1],
@@ -632,15 +660,42 @@ __device__ __forceinline__ void hn_stokes(const HermN &n, const double e1[4], co
   double Re1[4], Re2[4], Se1[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    Re1[k] = R[k][0] * e1[0] + R[k][1] * e1[1] + R[k][2] * e1[2] + R[k][3] * e1[3];
-    Re2[k] = R[k][0] * e2[0] + R[k][1] * e2[1] + R[k][2] * e2[2] + R[k][3] * e2[3];
-    Se1[k] = S[k][0] * e1[0] + S[k][1] * e1[1] + S[k][2] * e1[2] + S[k][3] * e1[3];
+    Re1[k] = dot4_rn(R[k], e1);
+    Re2[k] = dot4_rn(R[k], e2);
+    Se1[k] = dot4_rn(S[k], e1);
   }
-  *T11 = e1[0] * Re1[0] + e1[1] * Re1[1] + e1[2] * Re1[2] + e1[3] * Re1[3];
-  *T22 = e2[0] * Re2[0] + e2[1] * Re2[1] + e2[2] * Re2[2] + e2[3] * Re2[3];
-  *T12r = e1[0] * Re2[0] + e1[1] * Re2[1] + e1[2] * Re2[2] + e1[3] * Re2[3];
+  *T11 = sum4_rn(e1[0] * Re1[0], e1[1] * Re1[1], e1[2] * Re1[2], e1[3] * Re1[3]);
+  *T22 = sum4_rn(e2[0] * Re2[0], e2[1] * Re2[1], e2[2] * Re2[2], e2[3] * Re2[3]);
+  *T12r = sum4_rn(e1[0] * Re2[0], e1[1] * Re2[1], e1[2] * Re2[2], e1[3] * Re2[3]);
   /* Im T21 = e2 . S . e1 */
-  *T21i = e2[0] * Se1[0] + e2[1] * Se1[1] + e2[2] * Se1[2] + e2[3] * Se1[3];
+  *T21i = sum4_rn(e2[0] * Se1[0], e2[1] * Se1[1], e2[2] * Se1[2], e2[3] * Se1[3]);
+}
+
+/* One entry of N += Econ^T (new block - old block) Econ (stokes_to_tensor +
+ * complex_tetrad_to_coord_rank2, src/ipolarray.c:673-682, 730-748): exactly
+ * symmetric in (i, j) for the real part, antisymmetric for the imaginary */
+__device__ __forceinline__ double hn_upd_r(double r, double ai, double aj, double bi, double bj, double d11, double d22,
+                                           double dr12)
+{
+  const double w = __dadd_rn(__dmul_rn(ai, bj), __dmul_rn(bi, aj));
+  return __dadd_rn(r, __fma_rn(w, dr12, __fma_rn(__dmul_rn(ai, aj), d11, __dmul_rn(__dmul_rn(bi, bj), d22))));
+}
+__device__ __forceinline__ double hn_upd_s(double s, double ai, double aj, double bi, double bj, double di21)
+{
+  return __fma_rn(__dsub_rn(__dmul_rn(bi, aj), __dmul_rn(ai, bj)), di21, s);
+}
+__device__ __forceinline__ void hn_update(HermN *N, const double a[4], const double b[4], double d11, double d22,
+                                          double dr12, double di21)
+{
+#define UR(f, i, j) N->f = hn_upd_r(N->f, a[i], a[j], b[i], b[j], d11, d22, dr12)
+#define US(f, i, j) N->f = hn_upd_s(N->f, a[i], a[j], b[i], b[j], di21)
+  UR(r00, 0, 0); UR(r01, 0, 1); UR(r02, 0, 2); UR(r03, 0, 3);
+  UR(r11, 1, 1); UR(r12, 1, 2); UR(r13, 1, 3);
+  UR(r22, 2, 2); UR(r23, 2, 3); UR(r33, 3, 3);
+  US(s01, 0, 1); US(s02, 0, 2); US(s03, 0, 3);
+  US(s12, 1, 2); US(s13, 1, 3); US(s23, 2, 3);
+#undef UR
+#undef US
 }
 
 /* --------------------------------------------------------------------- */
@@ -1248,6 +1303,149 @@ __device__ __forceinline__ void absorb_emit(const JarT<R> &c, double x, R *SI, R
     *SQ = approximate_solve(SQ1, jQ, aI, jQ, aI, x, &tf);
     *SU = approximate_solve(SU1, jU, aI, jU, aI, x, &tf);
     *SV = approximate_solve(SV1, jV, aI, jV, aI, x, &tf);
+  }
+}
+
+/* The polarized step of evolve_N (Faraday half step, absorption/emission,
+ * Faraday half step, src/ipolarray.c:386-520) as the affine map
+ * S' = T S + u of the Stokes vector, for jU = aU = rU = 0.  T and u depend
+ * on the coefficients and the step length only, so a walk whose lanes share
+ * a ray computes them for many records side by side, off the chain of steps
+ * that carries S.  The formulas are those of faraday_apply and absorb_emit
+ * above, collected by the component of S they multiply. */
+struct StokesMap {
+  double T[16], u[4];
+};
+
+__device__ __forceinline__ void stokes_map(double jI, double jQ, double jV, double aI, double aQ, double aV, double rQ,
+                                           double rV, double x, StokesMap *m)
+{
+  /* Faraday half step: Q' = p Q - f U + q V, U' = f Q + c U - h V,
+   * V' = q Q + h U + s V */
+  double c = 1., ir = 0.5 * x, g = 0.;
+  const double rho2 = __fma_rn(rQ, rQ, __dmul_rn(rV, rV));
+  if (rho2 > IPG_CUT_PREVENT_NAN) {
+    const double rho = sqrt(rho2), irho = 1. / rho, ph = __dmul_rn(rho, 0.5 * x);
+    double s;
+    sincos(ph, &s, &c);
+    const double sh = sin(0.5 * ph);
+    ir = __dmul_rn(s, irho);
+    g = __dmul_rn(__dmul_rn(2. * sh, sh), __dmul_rn(irho, irho));
+  }
+  const double rQg = __dmul_rn(rQ, g);
+  const double p = __fma_rn(rQg, rQ, c), q = __dmul_rn(rQg, rV), s = __fma_rn(__dmul_rn(rV, g), rV, c);
+  const double f = __dmul_rn(rV, ir), h = __dmul_rn(rQ, ir);
+  /* absorption and emission: a symmetric matrix of I, Q, V; U decays alone */
+  double mII, mIQ = 0., mIV = 0., mQQ, mQV = 0., mVV, mUU, bI, bQ, bV;
+  const double aP2 = __fma_rn(aQ, aQ, __dmul_rn(aV, aV));
+  const double tauI = __dmul_rn(aI, x);
+  if (aP2 > IPG_CUT_PREVENT_NAN) {
+    const double aP = sqrt(aP2), tauP = __dmul_rn(aP, x);
+    const double adj = __fma_rn(aQ, jQ, __dmul_rn(aV, jV));
+    const double tm = __dsub_rn(tauI, tauP), tp = __dadd_rn(tauI, tauP);
+    const double efacm = exp(-tm), efacp = exp(-tp), efac = exp(-tauI);
+    const double iaP2 = 1. / aP2, i2aP2 = 0.5 * iaP2, i2aP = __dmul_rn(aP, i2aP2);
+    const double w = __dmul_rn(i2aP, __dsub_rn(efacp, efacm));
+    const double z = __fma_rn(i2aP2, __dadd_rn(efacm, efacp), -__dmul_rn(efac, iaP2));
+    mII = 0.5 * __dadd_rn(efacm, efacp);
+    mIQ = __dmul_rn(aQ, w);
+    mIV = __dmul_rn(aV, w);
+    const double zQ = __dmul_rn(z, aQ), zV = __dmul_rn(z, aV);
+    mQQ = __fma_rn(zQ, aQ, efac);
+    mQV = __dmul_rn(zQ, aV);
+    mVV = __fma_rn(zV, aV, efac);
+    mUU = efac;
+    double afacm = 1. - efacm, afac = 1. - efac, afacp = 1. - efacp;
+    /* 1 - e^-t by its series at small t (the last bits of 1 - e^-t) */
+    if (tm <= IPG_CUT_SMALL_TAU) {
+      afacm = __dmul_rn(tm, __fma_rn(-0.5 * tm, __fma_rn(tm, -(1. / 3.), 1.), 1.));
+      if (tauI <= IPG_CUT_SMALL_TAU) {
+        afac = __dmul_rn(tauI, __fma_rn(-0.5 * tauI, __fma_rn(tauI, -(1. / 3.), 1.), 1.));
+        if (tp <= IPG_CUT_SMALL_TAU) afacp = __dmul_rn(tp, __fma_rn(-0.5 * tp, __fma_rn(tp, -(1. / 3.), 1.), 1.));
+      }
+    }
+    const double iaI = 1. / aI, adjP = __dmul_rn(__dmul_rn(adj, iaI), iaP2);
+    const double iam = 1. / __dsub_rn(aI, aP), iap = 1. / __dadd_rn(aI, aP);
+    const double em = __dmul_rn(__fma_rn(aP, jI, -adj), iam), ep = __dmul_rn(__fma_rn(aP, jI, adj), iap);
+    const double gm = __dmul_rn(afacm, em), gp = __dmul_rn(afacp, ep);
+    bI = __dmul_rn(i2aP, __dadd_rn(gm, gp));
+    const double gd = __dmul_rn(i2aP2, __dsub_rn(gp, gm));
+    bQ = __fma_rn(afac, __fma_rn(jQ, iaI, -__dmul_rn(aQ, adjP)), __dmul_rn(aQ, gd));
+    bV = __fma_rn(afac, __fma_rn(jV, iaI, -__dmul_rn(aV, adjP)), __dmul_rn(aV, gd));
+  } else {
+    /* approximate_solve per component (constant j and a_I over the step) */
+    double e, wt;
+    if (tauI < 1.e-3) {
+      wt = __dmul_rn(x, __fma_rn(-0.5 * tauI, __fma_rn(tauI, -(1. / 3.), 1.), 1.));
+      e = __fma_rn(-aI, wt, 1.);
+    } else {
+      e = exp(-tauI);
+      wt = __dsub_rn(1., e) / aI;
+    }
+    mII = mQQ = mVV = mUU = e;
+    bI = __dmul_rn(jI, wt);
+    bQ = __dmul_rn(jQ, wt);
+    bV = __dmul_rn(jV, wt);
+  }
+  /* T = F M F, u = F b */
+  const double FQ[3] = {p, -f, q}, FU[3] = {f, c, -h}, FV[3] = {q, h, s};
+  double *T = m->T;
+  T[0] = mII;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double rQk = __fma_rn(mQQ, FQ[k], __dmul_rn(mQV, FV[k]));
+    const double rUk = __dmul_rn(mUU, FU[k]);
+    const double rVk = __fma_rn(mVV, FV[k], __dmul_rn(mQV, FQ[k]));
+    T[1 + k] = __fma_rn(mIQ, FQ[k], __dmul_rn(mIV, FV[k]));
+    T[5 + k] = __fma_rn(p, rQk, __fma_rn(-f, rUk, __dmul_rn(q, rVk)));
+    T[9 + k] = __fma_rn(f, rQk, __fma_rn(c, rUk, -__dmul_rn(h, rVk)));
+    T[13 + k] = __fma_rn(q, rQk, __fma_rn(h, rUk, __dmul_rn(s, rVk)));
+  }
+  T[4] = __fma_rn(p, mIQ, __dmul_rn(q, mIV));
+  T[8] = __fma_rn(f, mIQ, -__dmul_rn(h, mIV));
+  T[12] = __fma_rn(q, mIQ, __dmul_rn(s, mIV));
+  m->u[0] = bI;
+  m->u[1] = __fma_rn(p, bQ, __dmul_rn(q, bV));
+  m->u[2] = __fma_rn(f, bQ, -__dmul_rn(h, bV));
+  m->u[3] = __fma_rn(q, bQ, __dmul_rn(s, bV));
+}
+
+__device__ __forceinline__ double stokes_row(const double T[4], double u, double SI, double SQ, double SU, double SV)
+{
+  return __fma_rn(T[3], SV, __fma_rn(T[2], SU, __fma_rn(T[1], SQ, __fma_rn(T[0], SI, u))));
+}
+
+/* the step's Stokes floors (src/ipolarray.c:522-534) */
+__device__ __forceinline__ void stokes_floor(double *SI, double *SQ, double *SU, double *SV)
+{
+  if (*SI < 0) {
+    *SI = *SQ = *SU = *SV = 0;
+  } else {
+    double pf = sqrt(__fma_rn(*SV, *SV, __fma_rn(*SU, *SU, __dmul_rn(*SQ, *SQ)))) / *SI;
+    if (pf > 1.) {
+      *SQ /= pf;
+      *SU /= pf;
+      *SV /= pf;
+    }
+  }
+}
+
+/* The unpolarized step (approximate_solve, src/ipolarray.c:607-628) as
+ * I' = p I + q, with its optical depth */
+__device__ __forceinline__ void unpol_map(double ji, double ki, double jf, double kf, double dl, double *p, double *q,
+                                          double *dtau)
+{
+  const double javg = 0.5 * __dadd_rn(ji, jf), kavg = 0.5 * __dadd_rn(ki, kf);
+  const double t = __dmul_rn(dl, kavg);
+  *dtau = t;
+  if (t < 1.e-3) {
+    const double w = __dmul_rn(dl, __fma_rn(-0.5 * t, __fma_rn(t, -(1. / 3.), 1.), 1.));
+    *p = __fma_rn(-kavg, w, 1.);
+    *q = __dmul_rn(javg, w);
+  } else {
+    const double e = exp(-t);
+    *p = e;
+    *q = __dmul_rn(javg / kavg, __dsub_rn(1., e));
   }
 }
 

@@ -773,50 +773,17 @@ __device__ __forceinline__ void load_coef_m(const double *__restrict__ p, CoefBl
 __device__ __forceinline__ int evolve_N_coef(const CoefBlock &cb, double dlam, int zero_emission, HermN *N,
                                              double *tauF, int stokes_floors)
 {
-  Jar c;
-  c.jI = cb.jI;
-  c.jQ = cb.jQ;
-  c.jV = cb.jV;
-  c.aI = cb.aI;
-  c.aQ = cb.aQ;
-  c.aV = cb.aV;
-  c.rQ = cb.rQ;
-  c.rV = cb.rV;
-  c.jU = c.aU = c.rU = 0.;
-  if (zero_emission) c.jI = c.jQ = c.jU = c.jV = 0.;
+  StokesMap m;
+  stokes_map(zero_emission ? 0. : cb.jI, zero_emission ? 0. : cb.jQ, zero_emission ? 0. : cb.jV, cb.aI, cb.aQ, cb.aV,
+             cb.rQ, cb.rV, dlam, &m);
   double T11, T22, T12r, T21i;
   hn_stokes(*N, cb.e1, cb.e2, &T11, &T22, &T12r, &T21i);
-  double SI = (T11 + T22) / 2, SQ = (T11 - T22) / 2, SU = T12r, SV = T21i;
-  const FaradayRot R = faraday_rot(c.rQ, c.rU, c.rV, dlam * 0.5);
-  faraday_apply(R, c.rQ, c.rU, c.rV, &SQ, &SU, &SV);
-  absorb_emit(c, dlam, &SI, &SQ, &SU, &SV);
-  faraday_apply(R, c.rQ, c.rU, c.rV, &SQ, &SU, &SV);
-  *tauF += dlam * fabs(c.rV);
-  if (stokes_floors) {
-    if (SI < 0) {
-      SI = SQ = SU = SV = 0;
-    } else {
-      double pf = sqrt(SQ * SQ + SU * SU + SV * SV) / SI;
-      if (pf > 1.) {
-        SQ /= pf;
-        SU /= pf;
-        SV /= pf;
-      }
-    }
-  }
-  /* N += Econ^T (new block - old block) Econ (stokes_to_tensor +
-   * complex_tetrad_to_coord_rank2, src/ipolarray.c:673-682, 730-748) */
-  const double *a = cb.a, *b = cb.b;
-  double d11 = (SI + SQ) - T11, d22 = (SI - SQ) - T22, dr12 = SU - T12r, di21 = SV - T21i;
-#define DR(i, j) (a[i] * a[j] * d11 + b[i] * b[j] * d22 + (a[i] * b[j] + b[i] * a[j]) * dr12)
-#define DS(i, j) ((b[i] * a[j] - a[i] * b[j]) * di21)
-  N->r00 += DR(0, 0); N->r01 += DR(0, 1); N->r02 += DR(0, 2); N->r03 += DR(0, 3);
-  N->r11 += DR(1, 1); N->r12 += DR(1, 2); N->r13 += DR(1, 3);
-  N->r22 += DR(2, 2); N->r23 += DR(2, 3); N->r33 += DR(3, 3);
-  N->s01 += DS(0, 1); N->s02 += DS(0, 2); N->s03 += DS(0, 3);
-  N->s12 += DS(1, 2); N->s13 += DS(1, 3); N->s23 += DS(2, 3);
-#undef DR
-#undef DS
+  const double SI0 = (T11 + T22) / 2, SQ0 = (T11 - T22) / 2, SU0 = T12r, SV0 = T21i;
+  double SI = stokes_row(m.T, m.u[0], SI0, SQ0, SU0, SV0), SQ = stokes_row(m.T + 4, m.u[1], SI0, SQ0, SU0, SV0);
+  double SU = stokes_row(m.T + 8, m.u[2], SI0, SQ0, SU0, SV0), SV = stokes_row(m.T + 12, m.u[3], SI0, SQ0, SU0, SV0);
+  *tauF = __dadd_rn(*tauF, __dmul_rn(dlam, fabs(cb.rV)));
+  if (stokes_floors) stokes_floor(&SI, &SQ, &SU, &SV);
+  hn_update(N, cb.a, cb.b, (SI + SQ) - T11, (SI - SQ) - T22, SU - T12r, SV - T21i);
   int flag = 0;
   if (*tauF > 1.e100 || *tauF < -1.e100 || isnan(*tauF)) flag |= 2;
   if (isnan(N->r00) || isnan(SI)) flag |= 4;
@@ -824,6 +791,16 @@ __device__ __forceinline__ int evolve_N_coef(const CoefBlock &cb, double dlam, i
 }
 
 
+
+/* The FP32 step's scale factors are powers of two taken from a magnitude
+ * >= 1e-300: its exponent, and 2^e, straight from and to the bits (the
+ * library's ilogb and ldexp handle subnormals and specials, ~40 instructions
+ * each on the walk's chain). */
+__device__ __forceinline__ int pow2_exponent(double big)
+{
+  return min(((__double2hiint(big) >> 20) & 0x7ff) - 1023, 1022);
+}
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
 /* push_polar (src/ipolarray.c:253-289) with its increment in FP32, for the
  * FP32-step kernel: Mh is scaled by a power of two taken from its largest
@@ -834,8 +811,8 @@ __device__ __forceinline__ void hn_push_f32(const HermN &base, const HermN &Mh, 
                                             HermN *out)
 {
   const double big = fmax(fmax(fabs(Mh.r00), fabs(Mh.r11)), fmax(fmax(fabs(Mh.r22), fabs(Mh.r33)), 1e-300));
-  const int ex = ilogb(big);
-  const double sc = ldexp(1.0, -ex), us = ldexp(dl, ex);
+  const int ex = pow2_exponent(big);
+  const double sc = pow2(-ex), us = __dmul_rn(dl, pow2(ex));
   const float r00 = (float)(Mh.r00 * sc), r01 = (float)(Mh.r01 * sc), r02 = (float)(Mh.r02 * sc),
               r03 = (float)(Mh.r03 * sc), r11 = (float)(Mh.r11 * sc), r12 = (float)(Mh.r12 * sc),
               r13 = (float)(Mh.r13 * sc), r22 = (float)(Mh.r22 * sc), r23 = (float)(Mh.r23 * sc),
@@ -854,25 +831,25 @@ __device__ __forceinline__ void hn_push_f32(const HermN &base, const HermN &Mh, 
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      AR[i][j] = Af[i][0] * R[0][j] + Af[i][1] * R[1][j] + Af[i][2] * R[2][j] + Af[i][3] * R[3][j];
-      AS[i][j] = Af[i][0] * S[0][j] + Af[i][1] * S[1][j] + Af[i][2] * S[2][j] + Af[i][3] * S[3][j];
+      AR[i][j] = dot4f_rn(Af[i][0], Af[i][1], Af[i][2], Af[i][3], R[0][j], R[1][j], R[2][j], R[3][j]);
+      AS[i][j] = dot4f_rn(Af[i][0], Af[i][1], Af[i][2], Af[i][3], S[0][j], S[1][j], S[2][j], S[3][j]);
     }
-  out->r00 = base.r00 - us * (double)(AR[0][0] + AR[0][0]);
-  out->r01 = base.r01 - us * (double)(AR[0][1] + AR[1][0]);
-  out->r02 = base.r02 - us * (double)(AR[0][2] + AR[2][0]);
-  out->r03 = base.r03 - us * (double)(AR[0][3] + AR[3][0]);
-  out->r11 = base.r11 - us * (double)(AR[1][1] + AR[1][1]);
-  out->r12 = base.r12 - us * (double)(AR[1][2] + AR[2][1]);
-  out->r13 = base.r13 - us * (double)(AR[1][3] + AR[3][1]);
-  out->r22 = base.r22 - us * (double)(AR[2][2] + AR[2][2]);
-  out->r23 = base.r23 - us * (double)(AR[2][3] + AR[3][2]);
-  out->r33 = base.r33 - us * (double)(AR[3][3] + AR[3][3]);
-  out->s01 = base.s01 - us * (double)(AS[0][1] - AS[1][0]);
-  out->s02 = base.s02 - us * (double)(AS[0][2] - AS[2][0]);
-  out->s03 = base.s03 - us * (double)(AS[0][3] - AS[3][0]);
-  out->s12 = base.s12 - us * (double)(AS[1][2] - AS[2][1]);
-  out->s13 = base.s13 - us * (double)(AS[1][3] - AS[3][1]);
-  out->s23 = base.s23 - us * (double)(AS[2][3] - AS[3][2]);
+  out->r00 = __fma_rn(-us, (double)(AR[0][0] + AR[0][0]), base.r00);
+  out->r01 = __fma_rn(-us, (double)(AR[0][1] + AR[1][0]), base.r01);
+  out->r02 = __fma_rn(-us, (double)(AR[0][2] + AR[2][0]), base.r02);
+  out->r03 = __fma_rn(-us, (double)(AR[0][3] + AR[3][0]), base.r03);
+  out->r11 = __fma_rn(-us, (double)(AR[1][1] + AR[1][1]), base.r11);
+  out->r12 = __fma_rn(-us, (double)(AR[1][2] + AR[2][1]), base.r12);
+  out->r13 = __fma_rn(-us, (double)(AR[1][3] + AR[3][1]), base.r13);
+  out->r22 = __fma_rn(-us, (double)(AR[2][2] + AR[2][2]), base.r22);
+  out->r23 = __fma_rn(-us, (double)(AR[2][3] + AR[3][2]), base.r23);
+  out->r33 = __fma_rn(-us, (double)(AR[3][3] + AR[3][3]), base.r33);
+  out->s01 = __fma_rn(-us, (double)(AS[0][1] - AS[1][0]), base.s01);
+  out->s02 = __fma_rn(-us, (double)(AS[0][2] - AS[2][0]), base.s02);
+  out->s03 = __fma_rn(-us, (double)(AS[0][3] - AS[3][0]), base.s03);
+  out->s12 = __fma_rn(-us, (double)(AS[1][2] - AS[2][1]), base.s12);
+  out->s13 = __fma_rn(-us, (double)(AS[1][3] - AS[3][1]), base.s13);
+  out->s23 = __fma_rn(-us, (double)(AS[2][3] - AS[3][2]), base.s23);
 }
 
 /* (1 - e^-t) / t, bounded for every t (its limit 1 at t = 0) */
@@ -891,119 +868,157 @@ __device__ __forceinline__ float one_minus_exp_over(float t)
  * exact).  The Faraday angle is reduced modulo 2 pi in FP64 before its FP32
  * sine and cosine.  The N to Stokes projection and the update of N stay
  * FP64, so the accumulation along the ray is FP64. */
-__device__ __forceinline__ int evolve_N_coef_f32(const CoefBlock &cb, double dlam, int zero_emission, HermN *N,
-                                              double *tauF, int stokes_floors)
+/* the factors of that step that do not depend on S */
+struct StepF32 {
+  float fc, fs, fg, nQ, nV;                          /* Faraday half step */
+  float tI, tQ, tV, tP, itP2, ih, em, ep, e0, q0, qm, qp; /* absorption and emission */
+  int pol;                                           /* the polarized form of the absorption */
+  double jxI, jxQ, jxV;                              /* emission j dl */
+};
+
+__device__ __forceinline__ void step_f32_factors(double cjI, double cjQ, double cjV, double caI, double caQ, double caV,
+                                                 double crQ, double crV, double dlam, StepF32 *F)
 {
-  double T11, T22, T12r, T21i;
-  hn_stokes(*N, cb.e1, cb.e2, &T11, &T22, &T12r, &T21i);
-  const double SId = (T11 + T22) / 2, SQd = (T11 - T22) / 2, SUd = T12r, SVd = T21i;
-  const double jxId = zero_emission ? 0. : cb.jI * dlam, jxQd = zero_emission ? 0. : cb.jQ * dlam,
-               jxVd = zero_emission ? 0. : cb.jV * dlam;
-  const int ex = ilogb(fmax(fmax(fabs(SId), fabs(jxId)), 1e-300));
-  const double sc = ldexp(1.0, -ex);
-  float SI = (float)(SId * sc), SQ = (float)(SQd * sc), SU = (float)(SUd * sc), SV = (float)(SVd * sc);
-  const float jI = (float)(jxId * sc), jQ = (float)(jxQd * sc), jV = (float)(jxVd * sc);
+  F->jxI = __dmul_rn(cjI, dlam);
+  F->jxQ = __dmul_rn(cjQ, dlam);
+  F->jxV = __dmul_rn(cjV, dlam);
   /* Faraday half step (rU = 0): S turns about r by rho dl / 2 */
-  const double rho2 = cb.rQ * cb.rQ + cb.rV * cb.rV;
-  float fc, fs, fg, nQ, nV;
+  const double rho2 = __fma_rn(crQ, crQ, __dmul_rn(crV, crV));
   if (rho2 > IPG_CUT_PREVENT_NAN) {
-    const double rho = sqrt(rho2), phi = rho * dlam * 0.5;
+    const double rho = sqrt(rho2), phi = __dmul_rn(__dmul_rn(rho, dlam), 0.5);
     const float ph = (float)remainder(phi, 2. * IPG_PI);
     float sh = sinf(0.5f * ph);
-    sincosf(ph, &fs, &fc);
-    fg = 2.f * sh * sh;
-    nQ = (float)(cb.rQ / rho);
-    nV = (float)(cb.rV / rho);
+    sincosf(ph, &F->fs, &F->fc);
+    F->fg = 2.f * sh * sh;
+    F->nQ = (float)(crQ / rho);
+    F->nV = (float)(crV / rho);
   } else {
     /* the linear form: c = 1, no axial term, sin(rho x) / rho = x */
-    fc = 1.f;
-    fg = 0.f;
-    fs = 1.f;
-    nQ = (float)(cb.rQ * dlam * 0.5);
-    nV = (float)(cb.rV * dlam * 0.5);
+    F->fc = 1.f;
+    F->fg = 0.f;
+    F->fs = 1.f;
+    F->nQ = (float)(crQ * dlam * 0.5);
+    F->nV = (float)(crV * dlam * 0.5);
   }
-  auto faraday = [&](float &Q, float &U, float &V) {
-    const float Q0 = Q, U0 = U, V0 = V;
-    const float f = (nQ * Q0 + nV * V0) * fg;
-    Q = Q0 * fc + nQ * f - nV * U0 * fs;
-    U = U0 * fc + (nV * Q0 - nQ * V0) * fs;
-    V = V0 * fc + nV * f + nQ * U0 * fs;
-  };
-  faraday(SQ, SU, SV);
   /* absorption and emission over dl (aU = jU = 0).  The polarized form
    * divides by tau_P^2; below tau_P^2 = 1e-30 (where its FP32 square would
    * leave the normal range) the polarization coupling is negligible against
    * FP32's precision and the step takes the unpolarized-absorption form, as
    * the FP64 step does below alpha_P^2 = 1e-80 */
-  const double tP2d = (cb.aQ * cb.aQ + cb.aV * cb.aV) * dlam * dlam;
-  const float tI = (float)(cb.aI * dlam), tQ = (float)(cb.aQ * dlam), tV = (float)(cb.aV * dlam);
-  if (tP2d > 1e-30) {
-    const float tP2 = tQ * tQ + tV * tV, tP = sqrtf(tP2), itP2 = 1.f / tP2, ih = 0.5f / tP;
-    const float ads0 = tQ * SQ + tV * SV, adj = tQ * jQ + tV * jV;
-    const float em = expf(-(tI - tP)), ep = expf(-(tI + tP)), e0 = expf(-tI);
-    float SI2 = em * (0.5f * SI - ads0 * ih) + ep * (0.5f * SI + ads0 * ih);
-    const float cm = (-SI * tP + ads0) * (0.5f * itP2), cp = (SI * tP + ads0) * (0.5f * itP2);
-    float SQ2 = em * tQ * cm + ep * tQ * cp + e0 * (SQ - ads0 * tQ * itP2);
-    float SU2 = e0 * SU;
-    float SV2 = em * tV * cm + ep * tV * cp + e0 * (SV - ads0 * tV * itP2);
-    const float q0 = one_minus_exp_over(tI), qm = one_minus_exp_over(tI - tP), qp = one_minus_exp_over(tI + tP);
-    const float adjP = adj * itP2;
-    SQ2 += q0 * (jQ - tQ * adjP);
-    SV2 += q0 * (jV - tV * adjP);
-    SI2 += qm * (0.5f * jI - adj * ih) + qp * (0.5f * jI + adj * ih);
-    const float m2 = qm * (-tP * jI + adj) * (0.5f * itP2), p2 = qp * (tP * jI + adj) * (0.5f * itP2);
-    SQ2 += tQ * (m2 + p2);
-    SV2 += tV * (m2 + p2);
+  const double tP2d = __dmul_rn(__dmul_rn(__fma_rn(caQ, caQ, __dmul_rn(caV, caV)), dlam), dlam);
+  F->tI = (float)(caI * dlam);
+  F->tQ = (float)(caQ * dlam);
+  F->tV = (float)(caV * dlam);
+  F->pol = tP2d > 1e-30;
+  F->tP = F->itP2 = F->ih = F->em = F->ep = F->qm = F->qp = 0.f;
+  const float tI = F->tI, tQ = F->tQ, tV = F->tV;
+  if (F->pol) {
+    const float tP2 = __fmaf_rn(tQ, tQ, __fmul_rn(tV, tV)), tP = sqrtf(tP2);
+    F->tP = tP;
+    F->itP2 = 1.f / tP2;
+    F->ih = 0.5f / tP;
+    F->em = expf(-(tI - tP));
+    F->ep = expf(-(tI + tP));
+    F->e0 = expf(-tI);
+    F->q0 = one_minus_exp_over(tI);
+    F->qm = one_minus_exp_over(tI - tP);
+    F->qp = one_minus_exp_over(tI + tP);
+  } else {
+    F->e0 = (tI < 1e-3f) ? 0.f : expf(-tI);
+    F->q0 = (tI < 1e-3f) ? 0.f : one_minus_exp_over(tI);
+  }
+}
+
+/* S after the step, from S before it: the step's FP32 arithmetic, with its
+ * roundings spelled out (the walks that inline it must agree in every bit) */
+__device__ __forceinline__ void step_f32_apply(const StepF32 &F, double SId, double SQd, double SUd, double SVd,
+                                               double *SIo, double *SQo, double *SUo, double *SVo)
+{
+  const int ex = pow2_exponent(fmax(fmax(fabs(SId), fabs(F.jxI)), 1e-300));
+  const double sc = pow2(-ex);
+  float SI = (float)(SId * sc), SQ = (float)(SQd * sc), SU = (float)(SUd * sc), SV = (float)(SVd * sc);
+  const float jI = (float)(F.jxI * sc), jQ = (float)(F.jxQ * sc), jV = (float)(F.jxV * sc);
+  const float fc = F.fc, fs = F.fs, fg = F.fg, nQ = F.nQ, nV = F.nV;
+#define FM(a, b) __fmul_rn(a, b)
+#define FF(a, b, c) __fmaf_rn(a, b, c)
+#define SUM2(a, b, c, d) FF(a, b, FM(c, d)) /* a b + c d */
+  auto faraday = [&](float &Q, float &U, float &V) {
+    const float Q0 = Q, U0 = U, V0 = V;
+    const float f = FM(SUM2(nQ, Q0, nV, V0), fg);
+    Q = FF(-FM(nV, U0), fs, SUM2(Q0, fc, nQ, f));
+    const float d = FF(nV, Q0, -FM(nQ, V0));
+    U = SUM2(U0, fc, d, fs);
+    V = FF(FM(nQ, U0), fs, SUM2(V0, fc, nV, f));
+  };
+  faraday(SQ, SU, SV);
+  const float tI = F.tI, tQ = F.tQ, tV = F.tV;
+  if (F.pol) {
+    const float tP = F.tP, itP2 = F.itP2, ih = F.ih, hP = 0.5f * itP2;
+    const float ads0 = SUM2(tQ, SQ, tV, SV), adj = SUM2(tQ, jQ, tV, jV);
+    const float em = F.em, ep = F.ep, e0 = F.e0;
+    const float sm = __fsub_rn(0.5f * SI, FM(ads0, ih));
+    const float sp = __fadd_rn(0.5f * SI, FM(ads0, ih));
+    float SI2 = SUM2(em, sm, ep, sp);
+    const float cm = FM(FF(-SI, tP, ads0), hP), cp = FM(FF(SI, tP, ads0), hP);
+    float SQ2 = FF(e0, FF(-FM(ads0, tQ), itP2, SQ), SUM2(FM(em, tQ), cm, FM(ep, tQ), cp));
+    float SU2 = FM(e0, SU);
+    float SV2 = FF(e0, FF(-FM(ads0, tV), itP2, SV), SUM2(FM(em, tV), cm, FM(ep, tV), cp));
+    const float q0 = F.q0, qm = F.qm, qp = F.qp;
+    const float adjP = FM(adj, itP2);
+    SQ2 = FF(q0, FF(-tQ, adjP, jQ), SQ2);
+    SV2 = FF(q0, FF(-tV, adjP, jV), SV2);
+    const float jm = __fsub_rn(0.5f * jI, FM(adj, ih));
+    const float jp = __fadd_rn(0.5f * jI, FM(adj, ih));
+    SI2 = __fadd_rn(SI2, SUM2(qm, jm, qp, jp));
+    const float xm = FM(qm, FF(-tP, jI, adj)), xp = FM(qp, FF(tP, jI, adj));
+    const float mp2 = SUM2(xm, hP, xp, hP);
     SI = SI2;
-    SQ = SQ2;
+    SQ = FF(tQ, mp2, SQ2);
     SU = SU2;
-    SV = SV2;
+    SV = FF(tV, mp2, SV2);
   } else {
     /* approximate_solve per component with constant j and alpha_I */
     if (tI < 1e-3f) {
-      const float w = 1.f - (0.5f * tI) * (1.f - tI * (1.f / 3.f));
-      SI += (jI - SI * tI) * w;
-      SQ += (jQ - SQ * tI) * w;
-      SU += (0.f - SU * tI) * w;
-      SV += (jV - SV * tI) * w;
+      const float w = FF(-(0.5f * tI), FF(-tI, 1.f / 3.f, 1.f), 1.f);
+      SI = FF(FF(-SI, tI, jI), w, SI);
+      SQ = FF(FF(-SQ, tI, jQ), w, SQ);
+      SU = FF(FM(-SU, tI), w, SU);
+      SV = FF(FF(-SV, tI, jV), w, SV);
     } else {
-      const float e0 = expf(-tI), q0 = one_minus_exp_over(tI);
-      SI = SI * e0 + jI * q0;
-      SQ = SQ * e0 + jQ * q0;
-      SU = SU * e0;
-      SV = SV * e0 + jV * q0;
+      const float e0 = F.e0, q0 = F.q0;
+      SI = FF(SI, e0, FM(jI, q0));
+      SQ = FF(SQ, e0, FM(jQ, q0));
+      SU = FM(SU, e0);
+      SV = FF(SV, e0, FM(jV, q0));
     }
   }
   faraday(SQ, SU, SV);
-  *tauF += dlam * fabs(cb.rV);
-  const double is = ldexp(1.0, ex);
-  double SIo = SI * is, SQo = SQ * is, SUo = SU * is, SVo = SV * is;
-  if (stokes_floors) {
-    if (SIo < 0) {
-      SIo = SQo = SUo = SVo = 0;
-    } else {
-      double pf = sqrt(SQo * SQo + SUo * SUo + SVo * SVo) / SIo;
-      if (pf > 1.) {
-        SQo /= pf;
-        SUo /= pf;
-        SVo /= pf;
-      }
-    }
-  }
-  const double *a = cb.a, *b = cb.b;
-  double d11 = (SIo + SQo) - T11, d22 = (SIo - SQo) - T22, dr12 = SUo - T12r, di21 = SVo - T21i;
-#define DR(i, j) (a[i] * a[j] * d11 + b[i] * b[j] * d22 + (a[i] * b[j] + b[i] * a[j]) * dr12)
-#define DS(i, j) ((b[i] * a[j] - a[i] * b[j]) * di21)
-  N->r00 += DR(0, 0); N->r01 += DR(0, 1); N->r02 += DR(0, 2); N->r03 += DR(0, 3);
-  N->r11 += DR(1, 1); N->r12 += DR(1, 2); N->r13 += DR(1, 3);
-  N->r22 += DR(2, 2); N->r23 += DR(2, 3); N->r33 += DR(3, 3);
-  N->s01 += DS(0, 1); N->s02 += DS(0, 2); N->s03 += DS(0, 3);
-  N->s12 += DS(1, 2); N->s13 += DS(1, 3); N->s23 += DS(2, 3);
-#undef DR
-#undef DS
+#undef FM
+#undef FF
+#undef SUM2
+  const double is = pow2(ex);
+  *SIo = SI * is;
+  *SQo = SQ * is;
+  *SUo = SU * is;
+  *SVo = SV * is;
+}
+
+__device__ __forceinline__ int evolve_N_coef_f32(const CoefBlock &cb, double dlam, int zero_emission, HermN *N,
+                                              double *tauF, int stokes_floors)
+{
+  StepF32 F;
+  step_f32_factors(zero_emission ? 0. : cb.jI, zero_emission ? 0. : cb.jQ, zero_emission ? 0. : cb.jV, cb.aI, cb.aQ,
+                   cb.aV, cb.rQ, cb.rV, dlam, &F);
+  double T11, T22, T12r, T21i;
+  hn_stokes(*N, cb.e1, cb.e2, &T11, &T22, &T12r, &T21i);
+  double SI, SQ, SU, SV;
+  step_f32_apply(F, (T11 + T22) / 2, (T11 - T22) / 2, T12r, T21i, &SI, &SQ, &SU, &SV);
+  *tauF = __dadd_rn(*tauF, __dmul_rn(dlam, fabs(cb.rV)));
+  if (stokes_floors) stokes_floor(&SI, &SQ, &SU, &SV);
+  hn_update(N, cb.a, cb.b, (SI + SQ) - T11, (SI - SQ) - T22, SU - T12r, SV - T21i);
   int flag = 0;
   if (*tauF > 1.e100 || *tauF < -1.e100 || isnan(*tauF)) flag |= 2;
-  if (isnan(N->r00) || isnan(SIo)) flag |= 4;
+  if (isnan(N->r00) || isnan(SI)) flag |= 4;
   return flag;
 }
 
@@ -1140,8 +1155,10 @@ __device__ __forceinline__ void xfer_evolve(const DevCam &C, Lane &L, const Coef
     double jf = cb.ju, kf = cb.ku;
     L.js = jf;
     L.ks = kf;
-    if (zero_emission) L.I = approximate_solve(L.I, 0, ki, 0, kf, dl, &L.tau);
-    else L.I = approximate_solve(L.I, ji, ki, jf, kf, dl, &L.tau);
+    double ip, iq, dtau;
+    unpol_map(zero_emission ? 0. : ji, ki, zero_emission ? 0. : jf, kf, dl, &ip, &iq, &dtau);
+    L.I = __fma_rn(L.I, ip, iq);
+    L.tau = __dadd_rn(L.tau, dtau);
     if (!unpol) {
       L.flag |= flags >> 2;
       if constexpr (S32) L.flag |= evolve_N_coef_f32(cb, dl, zero_emission, &L.N, &L.tauF, C.stokes_floors);
@@ -1158,44 +1175,47 @@ __device__ __forceinline__ void xfer_step(const DevCam &C, Lane &L, const CoefBl
   xfer_evolve<S32>(C, L, cb, dl, unpol);
 }
 
-/* get_pixel's outputs at the end of a lane's walk: project_N
- * (src/ipolarray.c:578-598) in the camera's tetrad */
+/* get_pixel's outputs at the end of a ray's walk, from the Stokes sums of N
+ * in the camera's tetrad (project_N, src/ipolarray.c:578-598) */
+__device__ __forceinline__ void xfer_output(const DevCam &C, double I_unpol, double tau, double tauF, double T11,
+                                            double T22, double T12r, double T21i, int unpol, int nstep, int flag,
+                                            ipg_pixel_out *o)
+{
+  o->I_unpol = I_unpol;
+  o->tau = tau;
+  o->tauF = tauF;
+  o->I = o->Q = o->U = o->V = 0.;
+  if (!unpol) {
+    double Q = (T11 - T22) / 2, U = T12r;
+    /* the rotation by -2 rotcam with its roundings spelled out, so that
+     * every kernel that inlines this (the image, the batch, the adjoint's
+     * forward pass) gives the same bits whatever it contracts; + 0. makes
+     * every zero positive, whose sign depends on how a walk shares out the
+     * sums */
+    o->I = (T11 + T22) / 2 + 0.;
+    o->Q = __dadd_rn(__fma_rn(Q, C.cproj, -__dmul_rn(U, C.sproj)), 0.);
+    o->U = __dadd_rn(__fma_rn(Q, C.sproj, __dmul_rn(U, C.cproj)), 0.);
+    o->V = T21i + 0.;
+  }
+  o->nstep = nstep;
+  o->flag = flag;
+}
 template <class Lane>
 __device__ __forceinline__ void xfer_result(const DevCam &C, const Lane &L, int unpol, int nstep, ipg_pixel_out *o)
 {
-  o->I_unpol = L.I;
-  o->tau = L.tau;
-  o->tauF = L.tauF;
-  o->I = o->Q = o->U = o->V = 0.;
-  if (!unpol) {
-    /* project_N, src/ipolarray.c:578-598 */
-    double T11, T22, T12r, T21i;
-    hn_stokes(L.N, C.Ecov[1], C.Ecov[2], &T11, &T22, &T12r, &T21i);
-    double Q = (T11 - T22) / 2, U = T12r;
-    o->I = (T11 + T22) / 2;
-    /* the rotation by -2 rotcam with its roundings spelled out, so that
-     * every kernel that inlines this (the image, the batch, the adjoint's
-     * forward pass) gives the same bits whatever it contracts */
-    o->Q = fma(Q, C.cproj, -__dmul_rn(U, C.sproj));
-    o->U = fma(Q, C.sproj, __dmul_rn(U, C.cproj));
-    o->V = T21i;
-  }
-  o->nstep = nstep;
-  o->flag = L.flag;
+  double T11 = 0., T22 = 0., T12r = 0., T21i = 0.;
+  if (!unpol) hn_stokes(L.N, C.Ecov[1], C.Ecov[2], &T11, &T22, &T12r, &T21i);
+  xfer_output(C, L.I, L.tau, L.tauF, T11, T22, T12r, T21i, unpol, nstep, L.flag, o);
 }
 
 /* RM: the step-record layout, 0 FP64, 1 compact, -1 from the camera (the
  * no-alloc path) */
-/* CKK > 0 (the adjoint's forward pass): N of every step n with n % CKK == 0
- * is kept in ckpt, at entry (chunk * 32 + n % 32) / min(CKK, 32), so that
- * the adjoint recomputes N within a segment of CKK steps from its top. */
-template <int TPB = IPG_XFER_WIDE, int MINB = IPG_XFER_MINB, bool S32 = false, int RM = -1, int CKK = 0>
+template <int TPB = IPG_XFER_WIDE, int MINB = IPG_XFER_MINB, bool S32 = false, int RM = -1>
 __global__ void __launch_bounds__(TPB, MINB)
     k_transfer(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
                const int *__restrict__ chunk_prev, const RayRec *__restrict__ rays, ipg_pixel_out *__restrict__ out,
-               unsigned long long *__restrict__ counters, double *__restrict__ ckpt)
+               unsigned long long *__restrict__ counters)
 {
-  const DevGrid &G = c_grid;
   const DevCam &C = c_cam;
   const int unpol = C.unpol;
   XferLane L;
@@ -1209,16 +1229,6 @@ __global__ void __launch_bounds__(TPB, MINB)
       atomicAdd(&counters[CNT_RAD], (unsigned long long)L.nrad);
       has = xfer_fetch<RM>(L, list, n_list, pool, chunk_prev, rays, out, counters);
       continue;
-    }
-    if constexpr (CKK > 0) {
-      if (L.n % CKK == 0) {
-        constexpr int KC = CKK < IPG_CHUNK_STEPS ? CKK : IPG_CHUNK_STEPS;
-        double *q = ckpt + (((size_t)L.chunk * IPG_CHUNK_STEPS + L.n % IPG_CHUNK_STEPS) / KC) * 16;
-        store4(q, L.N.r00, L.N.r01, L.N.r02, L.N.r03);
-        store4(q + 4, L.N.r11, L.N.r12, L.N.r13, L.N.r22);
-        store4(q + 8, L.N.r23, L.N.r33, L.N.s01, L.N.s02);
-        store4(q + 12, L.N.s03, L.N.s12, L.N.s13, L.N.s23);
-      }
     }
     /* step n -> n-1 of integrate_emission's loop, src/ipolarray.c:78-244 */
     int s = L.n - 1;
@@ -1243,334 +1253,7 @@ __global__ void __launch_bounds__(TPB, MINB)
   }
 }
 
-/* ===================================================================== */
-/* k_transfer with its step records staged in shared memory               */
-/* ===================================================================== */
-/* k_transfer loads a step's record when the step starts, so each step
- * waits for a round trip to L2 or DRAM (long_scoreboard is its largest
- * stall).  Here every lane copies its next record into its own slots of
- * shared memory with cp.async while it computes the current one.
- *
- * One iteration consumes one record k: the transfer step k+1 -> k with k's
- * coefficient block (and record k+1's step length), then the push of N for
- * the step k -> k-1 with k's transport matrices (and k's step length).
- * That is k_transfer's sequence of operations, regrouped by record, so the
- * images are bit-identical.
- *
- * A record is copied in two parts, each issued as soon as the previous
- * record's part has been read from its slot: the coefficient block with the
- * tetrad rows (P1) and the transport matrices (P2).  A part's copy then
- * overlaps the other part's arithmetic.  With NBC = 2 the P1 part has two
- * slots and its copy is issued a whole iteration ahead.  Each lane's slots
- * are NBC P1 + P2 + 16 bytes apart: the 16-byte skew puts the lanes of a
- * quarter-warp in different banks. */
-template <int RM, int NBC>
-struct XStage {
-  static constexpr int P1_OFF = RM ? 128 : 256; /* byte offset of the coefficient block in the record */
-  static constexpr int P1 = RM ? 192 : 256;     /* coefficient block + tetrad rows */
-  static constexpr int P2 = RM ? 128 : 256;     /* transport matrices A1, A2 (from byte 0) */
-  static constexpr int LANE = NBC * P1 + P2 + 16; /* bytes of shared memory per lane */
-  static_assert(NBC == 1 || NBC == 2, "one or two coefficient slots");
-  static_assert(LANE % 16 == 0 && LANE % 128 == 16, "16-byte copies; quarter-warp lanes in distinct banks");
-  static_assert(IPG_XFER_WIDE * LANE <= 227 * 1024, "a wide block's slots fit an SM's shared memory");
-};
-/* slots per layout: FP64 records take one coefficient slot (528 bytes per
- * lane: three 128-lane blocks per SM, as many as the registers allow), the
- * compact records two (528 bytes as well) */
-template <int RM>
-struct XStageOf {
-  static constexpr int NBC = RM ? 2 : 1;
-  using T = XStage<RM, NBC>;
-};
-
-/* .ca: through L1, so the second 16 bytes of a 32-byte sector come from L1
- * instead of a second L2 request (with .cg the walk ran 30% slower) */
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
-{
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async_bytes(unsigned char *dst, const unsigned char *src)
-{
-#pragma unroll
-  for (int o = 0; o < BYTES; o += 16) cp_async16(dst + o, src + o);
-}
-
-template <int TPB = IPG_XFER_WIDE, int MINB = IPG_XFER_MINB, bool S32 = false, int RM = 0>
-__global__ void __launch_bounds__(TPB, MINB)
-    k_transfer_staged(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
-                      const int *__restrict__ chunk_prev, const RayRec *__restrict__ rays,
-                      ipg_pixel_out *__restrict__ out, unsigned long long *__restrict__ counters)
-{
-  static_assert(RM == 0 || RM == 1, "the staged walk is compiled per record layout");
-  using X = typename XStageOf<RM>::T;
-  constexpr int NBC = XStageOf<RM>::NBC;
-  extern __shared__ __align__(16) unsigned char xsm[];
-  unsigned char *slot_c = xsm + (size_t)threadIdx.x * X::LANE; /* NBC P1 slots */
-  unsigned char *slot_a = slot_c + NBC * X::P1;                /* one P2 slot */
-  const double *view_a = reinterpret_cast<const double *>(slot_a);
-  const DevCam &C = c_cam;
-  const int unpol = C.unpol;
-  XferLane L;
-  int n0 = 0;
-  /* a new ray: its top record's coefficients were read by xfer_fetch, so
-   * the first group is empty; the second copies the top record's matrices.
-   * In flight at the top of the iteration for record k, oldest first: k's
-   * P1 group, k's P2 group (NBC = 1: nothing else). */
-  auto start = [&]() {
-    n0 = L.n;
-    cp_async_commit();
-    if (!unpol && L.n > 0) cp_async_bytes<X::P2>(slot_a, reinterpret_cast<const unsigned char *>(L.rec_i));
-    cp_async_commit();
-  };
-  bool has = xfer_fetch<RM>(L, list, n_list, pool, chunk_prev, rays, out, counters);
-  if (has) start();
-  while (__any_sync(0xffffffffu, has)) {
-    if (!has) continue;
-    const int k = L.n;
-    const double *rec_f = nullptr; /* record k-1 */
-    if (k >= 1) {
-      const int s = k - 1;
-      if (s % IPG_CHUNK_STEPS == IPG_CHUNK_STEPS - 1) {
-        L.chunk = L.cprev;
-        L.cprev = chunk_prev[L.chunk];
-      }
-      rec_f = step_ptr(const_cast<double *>(pool), L.chunk, s % IPG_CHUNK_STEPS);
-      /* the record after it, into L2 */
-      if (s >= 1) {
-        if ((s - 1) % IPG_CHUNK_STEPS != IPG_CHUNK_STEPS - 1) prefetch_rec<RM>(rec_f - IPG_STEP_DOUBLES);
-        else if (L.cprev >= 0) prefetch_rec<RM>(step_ptr(const_cast<double *>(pool), L.cprev, IPG_CHUNK_STEPS - 1));
-      }
-    }
-    const unsigned char *src_c = reinterpret_cast<const unsigned char *>(rec_f) + X::P1_OFF;
-    if constexpr (NBC == 2) {
-      if (k >= 1) cp_async_bytes<X::P1>(slot_c + ((k - 1) & 1) * X::P1, src_c);
-      cp_async_commit();
-    }
-    /* the transfer step k+1 -> k (integrate_emission's loop,
-     * src/ipolarray.c:91-244) with record k's coefficients */
-    if (k < n0) {
-      if constexpr (NBC == 2) cp_async_wait<2>();
-      else cp_async_wait<1>();
-      CoefBlock cb;
-      const double *view_c = reinterpret_cast<const double *>(slot_c + (NBC == 2 ? (k & 1) : 0) * X::P1 - X::P1_OFF);
-      if constexpr (RM) load_coef_m(view_c, cb);
-      else load_coef(view_c, cb);
-      xfer_evolve<S32>(C, L, cb, L.dl_i, unpol);
-      L.dl_i = cb.dl;
-      L.nturns_i = cb.nturns;
-    }
-    if (k == 0) {
-      if constexpr (NBC == 1) cp_async_commit();
-      cp_async_commit();
-      ipg_pixel_out o;
-      xfer_result(C, L, unpol, rays[L.ray].nstep, &o);
-      out[L.ray] = o;
-      atomicAdd(&counters[CNT_RAD], (unsigned long long)L.nrad);
-      has = xfer_fetch<RM>(L, list, n_list, pool, chunk_prev, rays, out, counters);
-      if (has) start();
-      continue;
-    }
-    if constexpr (NBC == 1) {
-      cp_async_bytes<X::P1>(slot_c, src_c); /* the slot was read by the load above */
-      cp_async_commit();
-    }
-    /* push_polar for the step k -> k-1 with record k's matrices, then the
-     * copy of record k-1's matrices into the slot the push has read */
-    if (!unpol) {
-      cp_async_wait<1>();
-      xfer_push<S32, RM>(L, view_a, L.dl_i);
-      if (k >= 2) cp_async_bytes<X::P2>(slot_a, reinterpret_cast<const unsigned char *>(rec_f));
-    }
-    cp_async_commit();
-    L.rec_i = rec_f;
-    L.n = k - 1;
-  }
-  cp_async_wait<0>();
-}
-
-/* The same walk with each record part fetched by one bulk copy of the
- * tensor-memory-access unit (cp.async.bulk, completion on an mbarrier of the
- * lane's slot) instead of 16-byte copies through the load/store pipe: the
- * staged walk's largest stall is the shared-memory instruction queue (mio
- * throttle), which its 32 copies per step fill.  A slot's barrier flips its
- * phase when its copy has landed; before a slot is refilled, a proxy fence
- * orders the lane's reads of it before the copy's writes.  Every wait is
- * bounded: a copy that has not landed after IPG_XFER_BULK_SPINS polls sets
- * CNT_STALL and ends the lane, and the host reports the call as failed. */
-#ifndef IPG_XFER_BULK_SPINS
-#define IPG_XFER_BULK_SPINS (1u << 20)
-#endif
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bulk_fetch(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-/* waits for the barrier's phase `parity` to complete; false if it did not
- * within the bound */
-__device__ __forceinline__ bool bulk_wait(unsigned long long *bar, unsigned parity)
-{
-  for (unsigned it = 0; it < IPG_XFER_BULK_SPINS; it++) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void fence_slot_refill() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-/* CKK > 0 (the adjoint's forward pass): N at every record k with
- * k % CKK == 0, before the push k -> k-1, is kept in ckpt as by k_transfer */
-template <int TPB = IPG_XFER_WIDE, int MINB = IPG_XFER_MINB, bool S32 = false, int RM = 0, int CKK = 0>
-__global__ void __launch_bounds__(TPB, MINB)
-    k_transfer_bulk(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
-                    const int *__restrict__ chunk_prev, const RayRec *__restrict__ rays,
-                    ipg_pixel_out *__restrict__ out, unsigned long long *__restrict__ counters,
-                    double *__restrict__ ckpt = nullptr)
-{
-  static_assert(RM == 0 || RM == 1, "the staged walk is compiled per record layout");
-  using X = typename XStageOf<RM>::T;
-  constexpr int NBC = XStageOf<RM>::NBC;
-  extern __shared__ __align__(16) unsigned char xsm[];
-  __shared__ __align__(8) unsigned long long xbar[TPB][NBC + 1]; /* per lane: coefficient slot(s), matrices slot */
-  unsigned char *slot_c = xsm + (size_t)threadIdx.x * X::LANE;
-  unsigned char *slot_a = slot_c + NBC * X::P1;
-  const double *view_a = reinterpret_cast<const double *>(slot_a);
-  unsigned long long *bar = xbar[threadIdx.x];
-#pragma unroll
-  for (int j = 0; j <= NBC; j++)
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar + j)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  unsigned ph = 0;   /* phase parity of each barrier */
-  unsigned pend = 0; /* barriers with a copy issued and not yet waited for */
-  const DevCam &C = c_cam;
-  const int unpol = C.unpol;
-  XferLane L;
-  int n0 = 0;
-  bool has = xfer_fetch<RM>(L, list, n_list, pool, chunk_prev, rays, out, counters);
-  auto fetch = [&](void *dst, const void *src, unsigned bytes, int j) {
-    bulk_fetch(dst, src, bytes, bar + j);
-    pend |= 1u << j;
-  };
-  auto wait = [&](int j) {
-    bool ok = bulk_wait(bar + j, (ph >> j) & 1);
-    ph ^= 1u << j;
-    pend &= ~(1u << j);
-    return ok;
-  };
-  auto start = [&]() {
-    n0 = L.n;
-    if (!unpol && L.n > 0) fetch(slot_a, L.rec_i, X::P2, NBC);
-  };
-  /* a copy that did not land: flag it, give the lane's other copies in
-   * flight their bounded wait, and end the lane */
-  auto stall = [&]() {
-    atomicAdd(&counters[CNT_STALL], 1ULL);
-    for (int j = 0; j <= NBC; j++)
-      if (pend & (1u << j)) wait(j);
-    has = false;
-  };
-  if (has) start();
-  while (__any_sync(0xffffffffu, has)) {
-    if (!has) continue;
-    const int k = L.n;
-    const int chunk_k = L.chunk; /* record k's chunk */
-    const double *rec_f = nullptr; /* record k-1 */
-    if (k >= 1) {
-      const int s = k - 1;
-      if (s % IPG_CHUNK_STEPS == IPG_CHUNK_STEPS - 1) {
-        L.chunk = L.cprev;
-        L.cprev = chunk_prev[L.chunk];
-      }
-      rec_f = step_ptr(const_cast<double *>(pool), L.chunk, s % IPG_CHUNK_STEPS);
-      if (s >= 1) {
-        if ((s - 1) % IPG_CHUNK_STEPS != IPG_CHUNK_STEPS - 1) prefetch_rec<RM>(rec_f - IPG_STEP_DOUBLES);
-        else if (L.cprev >= 0) prefetch_rec<RM>(step_ptr(const_cast<double *>(pool), L.cprev, IPG_CHUNK_STEPS - 1));
-      }
-    }
-    const unsigned char *src_c = reinterpret_cast<const unsigned char *>(rec_f) + X::P1_OFF;
-    if constexpr (NBC == 2) {
-      if (k >= 1) {
-        fence_slot_refill();
-        fetch(slot_c + ((k - 1) & 1) * X::P1, src_c, X::P1, (k - 1) & 1);
-      }
-    }
-    /* the transfer step k+1 -> k with record k's coefficients */
-    if (k < n0) {
-      const int j = NBC == 2 ? (k & 1) : 0;
-      if (!wait(j)) {
-        stall();
-        continue;
-      }
-      CoefBlock cb;
-      const double *view_c = reinterpret_cast<const double *>(slot_c + j * X::P1 - X::P1_OFF);
-      if constexpr (RM) load_coef_m(view_c, cb);
-      else load_coef(view_c, cb);
-      xfer_evolve<S32>(C, L, cb, L.dl_i, unpol);
-      L.dl_i = cb.dl;
-      L.nturns_i = cb.nturns;
-    }
-    if (k == 0) {
-      ipg_pixel_out o;
-      xfer_result(C, L, unpol, rays[L.ray].nstep, &o);
-      out[L.ray] = o;
-      atomicAdd(&counters[CNT_RAD], (unsigned long long)L.nrad);
-      has = xfer_fetch<RM>(L, list, n_list, pool, chunk_prev, rays, out, counters);
-      if (has) start();
-      continue;
-    }
-    if constexpr (NBC == 1) {
-      fence_slot_refill(); /* the slot was read by the load above */
-      fetch(slot_c, src_c, X::P1, 0);
-    }
-    if constexpr (CKK > 0) {
-      if (k % CKK == 0) {
-        constexpr int KC = CKK < IPG_CHUNK_STEPS ? CKK : IPG_CHUNK_STEPS;
-        double *q = ckpt + (((size_t)chunk_k * IPG_CHUNK_STEPS + k % IPG_CHUNK_STEPS) / KC) * 16;
-        store4(q, L.N.r00, L.N.r01, L.N.r02, L.N.r03);
-        store4(q + 4, L.N.r11, L.N.r12, L.N.r13, L.N.r22);
-        store4(q + 8, L.N.r23, L.N.r33, L.N.s01, L.N.s02);
-        store4(q + 12, L.N.s03, L.N.s12, L.N.s13, L.N.s23);
-      }
-    }
-    /* push_polar for the step k -> k-1 with record k's matrices, then the
-     * fetch of record k-1's matrices into the slot the push has read */
-    if (!unpol) {
-      if (!wait(NBC)) {
-        stall();
-        continue;
-      }
-      xfer_push<S32, RM>(L, view_a, L.dl_i);
-      if (k >= 2) {
-        fence_slot_refill();
-        fetch(slot_a, rec_f, X::P2, NBC);
-      }
-    }
-    L.rec_i = rec_f;
-    L.n = k - 1;
-  }
-}
+#include "ipg_walk.cuh"
 
 /* ===================================================================== */
 /* longest-first order                                                    */
@@ -1709,7 +1392,7 @@ struct ipg_ctx {
   int32_t *d_pred;   /* predicted step counts (list positions), also staging */
   int *d_len_hist;   /* LEN_BUCKETS counters of the sort */
   int split;         /* 1: split waves into long and short batches */
-  int xstage;        /* records of the walk: 0 global loads, 1 16-byte copies, 2 bulk copies, -1 per layout */
+  int xstage;        /* the transfer walk: 0 k_transfer (one lane per ray), -1 k_walk */
   int emission_type; /* of the camera being traced */
   int rec_mixed;     /* IPG_RECORDS_MIXED: compact step records */
   int step32;        /* IPG_STEP_FP32: the polarized step in FP32 */
@@ -1794,43 +1477,13 @@ extern "C" int ipg_create(ipg_ctx **out, int device, size_t pool_bytes)
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_cnt, (NB_MAX + 1) * CNT_N * sizeof(unsigned long long));
   ctx->split = 1;
   if (getenv("IPG_NO_SPLIT")) ctx->split = 0;
-  /* how the transfer walk reads its step records: by default staged in
-   * shared memory; for FP64 records by 16-byte copies in the longest length
-   * class (lower latency per step: its walk alone takes 50 ms against 65 ms
-   * with bulk copies) and by one bulk copy per record part in the others
-   * (higher throughput: the bulk class's walk alone 29 ms against 50 ms),
-   * for compact records by 16-byte copies in every class (measured a little
-   * faster on the 400x400 image); IPG_XFER_STAGE=0 loads them from global
-   * memory, =1 and =2 select the 16-byte and the bulk copies for every
-   * class */
+  /* IPG_XFER_STAGE=0 selects the transfer walk with one lane per ray
+   * (k_transfer); any other value the default, k_walk.  Both give the same
+   * bits. */
   {
     const char *xs = getenv("IPG_XFER_STAGE");
-    ctx->xstage = (xs && xs[0] >= '0' && xs[0] <= '2') ? xs[0] - '0' : -1;
+    ctx->xstage = (xs && xs[0] == '0') ? 0 : -1;
   }
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, false, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<0>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, true, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<0>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, false, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<1>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, true, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<1>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, false, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<0>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, true, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<0>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, false, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<1>::T::LANE);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void *)k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, true, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, IPG_XFER_WIDE * XStageOf<1>::T::LANE);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_len_hist, LEN_BUCKETS * sizeof(int));
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->n_sm, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) {
@@ -2140,6 +1793,53 @@ struct Batch {
   mutable int geo_blocks; /* the geodesic's grid, as launched */
 };
 
+/* Launch of the transfer walk over a ray list: G lanes per ray, as many as
+ * keep every ray resident at once, G = 4 beyond that.  A step costs the warp
+ * the same ~400 instructions whatever G is, and with more lanes per ray a
+ * warp steps fewer rays together: the 128x128 image's longest two classes
+ * (78 and 1385 rays) walk 11 ms with G = 32 and 16 against 17 ms with G = 4,
+ * its bulk (14 921 rays) 5 ms with G = 4 against 12 ms with G = 32. */
+template <int G, bool S32, int RM, int CKK>
+static int launch_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
+                         ipg_pixel_out *d_out, unsigned long long *cnt, double *ckpt, cudaStream_t stream)
+{
+  const void *fn = (const void *)k_walk<G, S32, RM, CKK>;
+  const size_t sm = WalkSm<G, RM>::BYTES;
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
+  k_walk<G, S32, RM, CKK><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, ctx->d_rays, d_out, cnt, ckpt);
+  CK(cudaGetLastError());
+  return IPG_OK;
+}
+
+template <bool S32, int RM, int CKK>
+static int launch_walk(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
+                       ipg_pixel_out *d_out, unsigned long long *cnt, double *ckpt, cudaStream_t stream)
+{
+  const size_t resident = (size_t)ctx->n_sm * 8; /* warps */
+  const int G = n <= resident ? 32 : n <= 2 * resident ? 16 : n <= 4 * resident ? 8 : 4;
+  switch (G) {
+    case 32: return launch_walk_g<32, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
+    case 16: return launch_walk_g<16, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
+    case 8: return launch_walk_g<8, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
+    default: return launch_walk_g<4, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
+  }
+}
+
+template <bool S32, int RM>
+static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
+{
+  if (ctx->xstage == 0) {
+    const int xthreads = b.wide ? IPG_XFER_WIDE : 128;
+    int tb = grid_blocks(ctx, (const void *)k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM>, xthreads, b.run);
+    k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM><<<tb, xthreads, 0, b.stream>>>(
+        b.list, (int)b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt);
+    CK(cudaGetLastError());
+    return IPG_OK;
+  }
+  return launch_walk<S32, RM, 0>(ctx, b.list, b.run, b.pool, b.chunk_prev, d_out, b.cnt, nullptr, b.stream);
+}
+
 template <int P>
 static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg_pixel_out *d_out)
 {
@@ -2148,7 +1848,7 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
    * for the others): classes that run side by side then share their
    * instructions instead of competing for instruction-cache space. */
   const int threads = 128;
-  const int gthreads = b.wide ? 256 : threads, xthreads = b.wide ? IPG_XFER_WIDE : threads;
+  const int gthreads = b.wide ? 256 : threads;
   CK(cudaEventRecord(b.ev[0], b.stream));
   int gb = grid_blocks(ctx, (const void *)k_geodesic<P, 256, IPG_GEO_MINB>, gthreads, b.run);
   if (b.started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;
@@ -2191,38 +1891,10 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[2], b.stream));
-  /* one compiled transfer per step arithmetic and record layout, each
-   * holding only its own paths */
-#define IPG_LAUNCH_XFER(S32, RM)                                                                              \
-  do {                                                                                                       \
-    const int xmode = ctx->xstage >= 0 ? ctx->xstage : ((RM || b.wide) ? 1 : 2);                             \
-    if (xmode == 2) {                                                                                        \
-      size_t sm = (size_t)xthreads * XStageOf<RM>::T::LANE;                                                  \
-      int tb = grid_blocks(ctx, (const void *)k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM>,        \
-                           xthreads, b.run, sm);                                                             \
-      k_transfer_bulk<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM><<<tb, xthreads, sm, b.stream>>>(               \
-          b.list, (int)b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt);                              \
-    } else if (xmode == 1) {                                                                                 \
-      size_t sm = (size_t)xthreads * XStageOf<RM>::T::LANE;                                                       \
-      int tb = grid_blocks(ctx, (const void *)k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM>,      \
-                           xthreads, b.run, sm);                                                             \
-      k_transfer_staged<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM><<<tb, xthreads, sm, b.stream>>>(             \
-          b.list, (int)b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt);                              \
-    } else {                                                                                                 \
-      int tb = grid_blocks(ctx, (const void *)k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM>, xthreads,  \
-                           b.run);                                                                           \
-      k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM><<<tb, xthreads, 0, b.stream>>>(                     \
-          b.list, (int)b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt, nullptr);                     \
-    }                                                                                                        \
-  } while (0)
-  if (ctx->step32) {
-    if (ctx->rec_mixed) IPG_LAUNCH_XFER(true, 1);
-    else IPG_LAUNCH_XFER(true, 0);
-  } else {
-    if (ctx->rec_mixed) IPG_LAUNCH_XFER(false, 1);
-    else IPG_LAUNCH_XFER(false, 0);
-  }
-#undef IPG_LAUNCH_XFER
+  int rc = ctx->step32 ? (ctx->rec_mixed ? launch_transfer<true, 1>(ctx, b, d_out) : launch_transfer<true, 0>(ctx, b, d_out))
+                       : (ctx->rec_mixed ? launch_transfer<false, 1>(ctx, b, d_out)
+                                         : launch_transfer<false, 0>(ctx, b, d_out));
+  if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[3], b.stream));
   return IPG_OK;
@@ -2975,7 +2647,7 @@ extern "C" int ipg_trace_pixels_noalloc(const ipg_grid *g, const double *d_field
     NA_CK(cudaGetLastError());
     int tb = na_blocks(n_sm, (const void *)k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, false, 0>, threads, run);
     k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, false, 0><<<tb, threads, 0, stream>>>(list, (int)run, pool, chunk_prev,
-                                                                                   rays, d_out, cnt_d, nullptr);
+                                                                                   rays, d_out, cnt_d);
     NA_CK(cudaGetLastError());
     unsigned long long cnt[CNT_N];
     NA_CK(cudaMemcpyAsync(cnt, cnt_d, sizeof(cnt), cudaMemcpyDeviceToHost, stream));

@@ -516,6 +516,8 @@ __global__ void __launch_bounds__(TPB, MINB)
 }
 
 
+#include "ipg_geo_coop.cuh"
+
 /* Step count of each ray at a coarser accuracy (eps_scale x eps), without
  * storing anything: a cheap prediction of the ray lengths, so that the full
  * trace can start the longest rays first.  pred[t] is the count of list
@@ -1393,7 +1395,7 @@ struct ipg_ctx {
   int *d_len_hist;   /* LEN_BUCKETS counters of the sort */
   int split;         /* 1: split waves into long and short batches */
   int xstage;        /* the transfer walk: 0 k_transfer (one lane per ray), -1 k_walk */
-  int emission_type; /* of the camera being traced */
+  int emission_type, unpol; /* of the camera being traced */
   int rec_mixed;     /* IPG_RECORDS_MIXED: compact step records */
   int step32;        /* IPG_STEP_FP32: the polarized step in FP32 */
   int fits32;        /* IPG_FITS_FP32: the thermal fits with FP32 shapes */
@@ -1791,7 +1793,53 @@ struct Batch {
   cudaEvent_t coef_after; /* k_coeffs waits for this event (or none) */
   int *started;           /* device view of host flags: the geodesic's blocks mark their start (or none) */
   mutable int geo_blocks; /* the geodesic's grid, as launched */
+  int split;              /* a class of a split wave */
 };
+
+/* Rays up to which a launch gives each ray eight lanes (k_geodesic_coop):
+ * eight warps of four rays per SM, two per scheduler.  1 / 1024 / 4000 rays
+ * of a 400x400 camera take 5.4 / 13.3 / 16.3 ms against 9.7 / 24.2 / 30.0 ms
+ * with a lane per ray; with 14 000 rays beside a large wave it loses (the
+ * 400x400 image's middle class: 175 against 156 ms per image), since it
+ * executes twice the instructions per ray-step of full 32-ray warps. */
+static bool geo_coop(const ipg_ctx *ctx, int plug, size_t n) { return plug == IPG_PLUG_IHARM && n <= (size_t)ctx->n_sm * 32; }
+/* In a split wave its blocks are 384 threads wide (their registers fill an
+ * SM, so that no other class's kernel runs beside them and competes for
+ * instruction fetch: the 400x400 image 154 ms against 162 ms with 32-thread
+ * blocks); alone, 32-thread blocks spread the warps over all schedulers. */
+#define IPG_COOP_WIDE 384
+
+template <class CS>
+static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const int32_t *d_ij, const int32_t *list,
+                           size_t n, double *pool, int *chunk_prev, int2 *chunk_meta, long long n_chunks,
+                           unsigned long long *cnt, RayRec *rays, int32_t *deferred, const int32_t *grp,
+                           cudaStream_t stream, int *started, int *blocks)
+{
+#define IPG_LAUNCH_COOP(POL, MIXED, TPB)                                                                           \
+  do {                                                                                                             \
+    int gb = grid_blocks(ctx, (const void *)k_geodesic_coop<POL, MIXED, TPB, CS>, TPB, n * GC_LANES);              \
+    if (started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;                                                     \
+    *blocks = gb;                                                                                                  \
+    k_geodesic_coop<POL, MIXED, TPB, CS><<<gb, TPB, 0, stream>>>(d_ij, list, (int)n, pool, chunk_prev, chunk_meta, \
+                                                                 n_chunks, cnt, rays, deferred, grp, started);     \
+  } while (0)
+#define IPG_LAUNCH_COOP_T(POL, MIXED)                     \
+  do {                                                    \
+    if (wide) IPG_LAUNCH_COOP(POL, MIXED, IPG_COOP_WIDE); \
+    else IPG_LAUNCH_COOP(POL, MIXED, 32);                 \
+  } while (0)
+  if (unpol) {
+    if (mixed) IPG_LAUNCH_COOP_T(false, true);
+    else IPG_LAUNCH_COOP_T(false, false);
+  } else {
+    if (mixed) IPG_LAUNCH_COOP_T(true, true);
+    else IPG_LAUNCH_COOP_T(true, false);
+  }
+#undef IPG_LAUNCH_COOP_T
+#undef IPG_LAUNCH_COOP
+  CK(cudaGetLastError());
+  return IPG_OK;
+}
 
 /* Launch of the transfer walk over a ray list: G lanes per ray, as many as
  * keep every ray resident at once, G = 4 beyond that.  A step costs the warp
@@ -1850,12 +1898,19 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
   const int threads = 128;
   const int gthreads = b.wide ? 256 : threads;
   CK(cudaEventRecord(b.ev[0], b.stream));
-  int gb = grid_blocks(ctx, (const void *)k_geodesic<P, 256, IPG_GEO_MINB>, gthreads, b.run);
-  if (b.started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;
-  b.geo_blocks = gb;
-  k_geodesic<P, 256, IPG_GEO_MINB><<<gb, gthreads, 0, b.stream>>>(d_ij, b.list, (int)b.run, b.pool, b.chunk_prev,
-                                                                  b.chunk_meta, b.n_chunks, b.cnt, ctx->d_rays,
-                                                                  b.deferred, nullptr, b.started);
+  if (geo_coop(ctx, P, b.run)) {
+    int rc = launch_geo_coop<CamOne>(ctx, ctx->unpol, ctx->rec_mixed, b.split, d_ij, b.list, b.run, b.pool,
+                                     b.chunk_prev, b.chunk_meta, b.n_chunks, b.cnt, ctx->d_rays, b.deferred, nullptr,
+                                     b.stream, b.started, &b.geo_blocks);
+    if (rc) return rc;
+  } else {
+    int gb = grid_blocks(ctx, (const void *)k_geodesic<P, 256, IPG_GEO_MINB>, gthreads, b.run);
+    if (b.started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;
+    b.geo_blocks = gb;
+    k_geodesic<P, 256, IPG_GEO_MINB><<<gb, gthreads, 0, b.stream>>>(d_ij, b.list, (int)b.run, b.pool, b.chunk_prev,
+                                                                    b.chunk_meta, b.n_chunks, b.cnt, ctx->d_rays,
+                                                                    b.deferred, nullptr, b.started);
+  }
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[1], b.stream));
   if (b.coef_after) CK(cudaStreamWaitEvent(b.stream, b.coef_after, 0));
@@ -2102,6 +2157,7 @@ static int trace_core(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *d_ij, 
   make_devcam(cam, &dc);
   dc.mixed = ctx->rec_mixed;
   ctx->emission_type = cam->emission_type;
+  ctx->unpol = cam->only_unpolarized;
   CK(cudaMemcpyToSymbolAsync(c_grid, &ctx->dg, sizeof(DevGrid), 0, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyToSymbolAsync(c_plug, &ctx->dp, sizeof(DevPlug), 0, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyToSymbolAsync(c_cam, &dc, sizeof(DevCam), 0, cudaMemcpyHostToDevice, ctx->stream));
@@ -2165,10 +2221,14 @@ static int trace_core(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *d_ij, 
         bt[b].coef_after = nullptr;
         bt[b].started = (b == 0 && wide[0] && nb > 1) ? ctx->d_started : nullptr;
         bt[b].geo_blocks = 0;
+        bt[b].split = 1;
         /* the shorter classes' coefficient passes wait for the longest
          * class's geodesics: run beside them, they slow the longest rays'
-         * steps four- to eightfold (those rays' SMs hold no other block) */
-        if (IPG_COEF_WAIT_LONGEST && b > 0 && wide[0]) bt[b].coef_after = ctx->bev[0][1];
+         * steps four- to eightfold (those rays' SMs hold no other block).
+         * With eight lanes per ray those end before the others' geodesics
+         * do, and waiting for them gains nothing (400x400: 154 against 156
+         * ms). */
+        if (IPG_COEF_WAIT_LONGEST && b > 0 && wide[0] && !geo_coop(ctx, ctx->plug, sizes[0])) bt[b].coef_after = ctx->bev[0][1];
         c0 += ncb;
         r0 += sizes[b];
       }
@@ -2183,7 +2243,7 @@ static int trace_core(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *d_ij, 
         CK(cudaStreamWaitEvent(bt[b].stream, ctx->ev_fork, 0));
         rc = launch_batch(ctx, bt[b], d_ij, d_out);
         if (rc) return rc;
-        if (bt[b].started) wait_started(ctx, bt[b].geo_blocks);
+        if (bt[b].started && bt[b].geo_blocks) wait_started(ctx, bt[b].geo_blocks);
         CK(cudaEventRecord(ctx->ev_join[b], bt[b].stream));
         CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join[b], 0));
       }

@@ -267,9 +267,12 @@ int ipg_render_batch(ipg_ctx *ctx, const ipg_instance *inst, size_t n, ipg_insta
  * dL/d|B| for every ghost-padded cell of the uploaded iharm fields (the
  * cell values the trilinear gather reads, layout of ipg_upload_iharm).  The
  * call traces the pixels again (the forward outputs come back in out, when
- * non-NULL), keeps N every ckpt_interval steps (16, 32 or 64) and walks each
- * ray back to front, recomputing the coherency tensor between checkpoints
- * and the fits with their derivatives at every radiating step.  Geodesics
+ * non-NULL), leaves in each step record what the reverse walk needs of the
+ * step, and walks each ray from the camera to its source; the fits are
+ * re-evaluated with their derivatives at every radiating step.
+ * ckpt_interval (16, 32 or 64) is kept for callers that pass it: nothing is
+ * recomputed between checkpoints any more, and the gradients do not depend
+ * on it.  Geodesics
  * do not depend on the fluid and are not differentiated; neither are the
  * sigma cut and the host's Theta_e floor (zero derivative almost
  * everywhere).  Needs a polarized image without Stokes floors (IPG_E_ARG
@@ -346,8 +349,8 @@ typedef struct ipg_stats {
   double geodesic_span_ms;
   double coeffs_span_ms;
   double transfer_span_ms;
-  /* ipg_adjoint: the reverse walk (link pass and adjoint kernel) and the
-   * scatter of the cells' gradients; its forward pass is in geodesic_ms,
+  /* ipg_adjoint: the reverse walk (link pass and k_adj_walk) and the
+   * gradients of the coefficients and cells (k_adj_scatter); its forward pass is in geodesic_ms,
    * coeffs_ms and transfer_ms */
   double adjoint_ms;
   double adj_scatter_ms;

@@ -20,20 +20,15 @@
  * |B|) at the point and scatter-adds that to the eight cells of the
  * trilinear gather (src/grid.c:15-44), with their weights.
  *
- *   - The N it needs are recomputed, not stored: the forward pass keeps
- *     N every K steps (k_transfer with CKK = K), and the adjoint
- *     recomputes a segment from its top with the forward's own functions,
- *     so they are the forward's bits; it keeps, per step of the segment,
- *     N after the step's two pushes (the state evolve_N was applied to).
- *   - The walk (k_adjoint, one lane per ray) leaves dL/d(coefficients) at
- *     each radiating record; k_adj_scatter, one thread per record, turns
- *     them into dL/d(ne, Theta_e, |B|) and scatter-adds those to the cells,
- *     off the walk's critical path.
+ *   - The forward pass (k_walk, ADJ) leaves in each radiating record the
+ *     Stokes vector its step was applied to, so no N is kept or recomputed.
+ *   - The walk (k_adj_walk, four or more lanes per ray) carries dL/dN and
+ *     leaves dL/dS' of each radiating record's step; k_adj_scatter, one
+ *     thread per record, turns it into dL/d(coefficients) and dL/d(ne,
+ *     Theta_e, |B|) and scatter-adds those to the cells.
  *   - The coefficients' derivatives come from re-evaluating the fits
  *     (jar_fits) in forward-mode dual numbers along ne, Theta_e, |B|
- *     (ipg_dual.cuh), and the step's from re-evaluating the Faraday and
- *     absorption/emission step (faraday_rot, absorb_emit) in duals along
- *     the Stokes vector and the eight coefficients.
+ *     (ipg_dual.cuh), the step's from its transpose (stokes_step_vjp).
  *   - Gradients of N are kept as full-matrix gradients of its real
  *     (symmetric) and imaginary (antisymmetric) parts, upper triangles
  *     stored: every map here keeps those symmetries.
@@ -47,72 +42,6 @@
 
 #include "ipg_step_vjp.cuh"
 
-/* gradient of a Hermitian N: g.r[ij] = dL/dRe N[i][j] = dL/dRe N[j][i],
- * g.s[ij] = dL/dIm N[i][j] = -dL/dIm N[j][i] (the same layout as HermN) */
-typedef HermN GradN;
-
-__device__ __forceinline__ void gn_full(const GradN &g, double R[4][4], double S[4][4]) { hn_unpack(g, R, S); }
-
-__device__ __forceinline__ void gn_pack(const double R[4][4], const double S[4][4], GradN *g)
-{
-  g->r00 = R[0][0]; g->r01 = R[0][1]; g->r02 = R[0][2]; g->r03 = R[0][3];
-  g->r11 = R[1][1]; g->r12 = R[1][2]; g->r13 = R[1][3];
-  g->r22 = R[2][2]; g->r23 = R[2][3]; g->r33 = R[3][3];
-  g->s01 = S[0][1]; g->s02 = S[0][2]; g->s03 = S[0][3];
-  g->s12 = S[1][2]; g->s13 = S[1][3]; g->s23 = S[2][3];
-}
-
-/* base + s (A^T G + G A), the transpose of X -> A X + X A^T, for both parts */
-__device__ __forceinline__ void gn_push_adj(const GradN &base, const GradN &G, const double A[4][4], double s,
-                                            GradN *out)
-{
-  double R[4][4], S[4][4], oR[4][4], oS[4][4];
-  gn_full(G, R, S);
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      double ar = 0., as = 0., ra = 0., sa = 0.;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        ar += A[k][i] * R[k][j];
-        as += A[k][i] * S[k][j];
-        ra += R[i][k] * A[k][j];
-        sa += S[i][k] * A[k][j];
-      }
-      oR[i][j] = ar + ra;
-      oS[i][j] = as + sa;
-    }
-  double bR[4][4], bS[4][4];
-  gn_full(base, bR, bS);
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      oR[i][j] = bR[i][j] + s * oR[i][j];
-      oS[i][j] = bS[i][j] + s * oS[i][j];
-    }
-  gn_pack(oR, oS, out);
-}
-
-/* G += the transpose of hn_stokes at (gT11, gT22, gT12r, gT21i):
- * T11 = e1 R e1, T22 = e2 R e2, T12r = e1 R e2, T21i = e2 S e1 (symmetric
- * and antisymmetric parts of the outer products) */
-__device__ __forceinline__ void gn_add_stokes_adj(const double e1[4], const double e2[4], double g11, double g22,
-                                                  double g12r, double g21i, GradN *G)
-{
-  double R[4][4], S[4][4];
-  gn_full(*G, R, S);
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      R[i][j] += g11 * e1[i] * e1[j] + g22 * e2[i] * e2[j] + 0.5 * g12r * (e1[i] * e2[j] + e2[i] * e1[j]);
-      S[i][j] += 0.5 * g21i * (e2[i] * e1[j] - e1[i] * e2[j]);
-    }
-  gn_pack(R, S, G);
-}
-
 /* the polarized step S -> S' of evolve_N (Faraday half step, absorption and
  * emission, Faraday half step; src/ipolarray.c:390-520) in any number type */
 template <class R>
@@ -122,19 +51,6 @@ __device__ __forceinline__ void stokes_step(const JarT<R> &c, double dlam, R S[4
   faraday_apply(F, c.rQ, c.rU, c.rV, &S[1], &S[2], &S[3]);
   absorb_emit(c, dlam, &S[0], &S[1], &S[2], &S[3]);
   faraday_apply(F, c.rQ, c.rU, c.rV, &S[1], &S[2], &S[3]);
-}
-
-/* the coefficient block cb as the step reads it, with zero_emission */
-__device__ __forceinline__ void coef_values(const CoefBlock &cb, int zero_emission, double v[8])
-{
-  v[0] = zero_emission ? 0. : cb.jI;
-  v[1] = zero_emission ? 0. : cb.jQ;
-  v[2] = zero_emission ? 0. : cb.jV;
-  v[3] = cb.aI;
-  v[4] = cb.aQ;
-  v[5] = cb.aV;
-  v[6] = cb.rQ;
-  v[7] = cb.rV;
 }
 
 /* One pass of the step in Dual<4>: directions d0..d3 among the 12 inputs
@@ -167,64 +83,6 @@ __device__ __forceinline__ void step_vjp_pass(const double S0[4], const double c
   for (int d = 0; d < 4; d++) out[d] = u[0] * S[0].d[d] + u[1] * S[1].d[d] + u[2] * S[2].d[d] + u[3] * S[3].d[d];
 }
 
-/* The transpose of evolve_N_coef at N (the state it was applied to):
- * G (dL/dN after the step) becomes dL/dN before it, and gc[8] receives
- * dL/d(jI, jQ, jV, aI, aQ, aV, rQ, rV) (zero for the emissivities when the
- * step had zero_emission). */
-__device__ __forceinline__ void evolve_adj(const CoefBlock &cb, double dlam, int zero_emission, const HermN &N,
-                                           GradN *G, double gc[8])
-{
-  double T11, T22, T12r, T21i;
-  hn_stokes(N, cb.e1, cb.e2, &T11, &T22, &T12r, &T21i);
-  const double S0[4] = {(T11 + T22) / 2, (T11 - T22) / 2, T12r, T21i};
-  /* N' = N + D(d), d = (SI'+SQ' - T11, SI'-SQ' - T22, SU' - T12r, SV' - T21i) */
-  double R[4][4], Sg[4][4];
-  gn_full(*G, R, Sg);
-  const double *a = cb.a, *b = cb.b;
-  double aRa = 0., bRb = 0., aRb = 0., bSa = 0.;
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      aRa += a[i] * R[i][j] * a[j];
-      bRb += b[i] * R[i][j] * b[j];
-      aRb += a[i] * R[i][j] * b[j];
-      bSa += b[i] * Sg[i][j] * a[j];
-    }
-  const double g11 = aRa, g22 = bRb, g12 = 2. * aRb, g21 = 2. * bSa;
-  const double u[4] = {g11 + g22, g11 - g22, g12, g21};
-  double cv[8];
-  coef_values(cb, zero_emission, cv);
-  double gS[4];
-  stokes_step_vjp(cv, dlam, S0, u, gS, gc);
-  if (zero_emission) gc[0] = gc[1] = gc[2] = 0.;
-  /* d/dT: directly (-d) and through S = (T11+T22, T11-T22)/2, T12r, T21i */
-  const double t11 = -g11 + 0.5 * (gS[0] + gS[1]);
-  const double t22 = -g22 + 0.5 * (gS[0] - gS[1]);
-  const double t12 = -g12 + gS[2];
-  const double t21 = -g21 + gS[3];
-  gn_add_stokes_adj(cb.e1, cb.e2, t11, t22, t12, t21, G);
-}
-
-/* step records by step index, walking the ray's chunk chain both ways */
-struct ChunkWalk {
-  int chunk, base; /* chunk holding steps base .. base + 31 */
-};
-
-__device__ __forceinline__ const double *walk_rec(ChunkWalk &w, int n, const double *pool, const int *prev,
-                                                  const int *next)
-{
-  while (n < w.base) {
-    w.chunk = prev[w.chunk];
-    w.base -= IPG_CHUNK_STEPS;
-  }
-  while (n >= w.base + IPG_CHUNK_STEPS) {
-    w.chunk = next[w.chunk];
-    w.base += IPG_CHUNK_STEPS;
-  }
-  return step_ptr(const_cast<double *>(pool), w.chunk, n - w.base);
-}
-
 /* forward links of the chunk chains and each ray's first chunk */
 __global__ void k_adj_link(const int *__restrict__ prev, const int2 *__restrict__ meta,
                            const unsigned long long *__restrict__ counters, long long n_chunks, int *__restrict__ next,
@@ -237,32 +95,6 @@ __global__ void k_adj_link(const int *__restrict__ prev, const int2 *__restrict_
     if (p >= 0) next[p] = (int)c;
     else first[meta[c].x] = (int)c;
   }
-}
-
-/* one forward step n -> n-1 of N (the polarized part of xfer_step);
- * *Np receives N after the two pushes, before evolve_N */
-__device__ __forceinline__ void fwd_N(const DevCam &C, const double *rec_n, const double *rec_m, HermN *N,
-                                      HermN *Np)
-{
-  const DevGrid &G = c_grid;
-  const double dl = rec_n[REC_DL];
-  double A[4][4];
-  HermN Nh, Nn;
-  load_A(rec_n + REC_A1, A);
-  hn_push(*N, *N, A, (0.5 * dl) * G.inv_dlfac, &Nh);
-  load_A(rec_n + REC_A2, A);
-  hn_push(*N, Nh, A, dl * G.inv_dlfac, &Nn);
-  *Np = Nn;
-  CoefBlock cb;
-  load_coef(rec_m, cb);
-  const int flags = (int)cb.flags;
-  if (flags & 1) {
-    int zero_emission = (flags & 2) ? 1 : 0;
-    if (C.target_nturns >= 0 && (int)rec_n[REC_NTURNS] != C.target_nturns) zero_emission = 1;
-    double tauF = 0.;
-    evolve_N_coef(cb, dl, zero_emission, &Nn, &tauF, 0);
-  }
-  *N = Nn;
 }
 
 /* dL/d(ne, Theta_e, |B|) at the point of a radiating record from dL/d(its
@@ -314,101 +146,222 @@ __device__ __forceinline__ void fluid_scatter(const double *__restrict__ fields,
     }
 }
 
-/* One lane per ray of the wave: the adjoint walk, camera to source. */
-template <int K>
-__global__ void __launch_bounds__(128, 1)
-    k_adjoint(const int32_t *__restrict__ list, int n_list, double *__restrict__ pool,
-              const double *__restrict__ adj_side, const double *__restrict__ ckpt, const int *__restrict__ prev,
-              const int *__restrict__ next, const int *__restrict__ first, const RayRec *__restrict__ rays,
-              const double *__restrict__ dL_dout, const double *__restrict__ fields, double *__restrict__ g_ne,
-              double *__restrict__ g_th, double *__restrict__ g_b, unsigned long long *__restrict__ counter)
+/* The adjoint walk, camera to source, with G lanes per ray (the layout of
+ * k_walk: a warp walks 32/G rays over blocks of G records).  Step n = k + 1
+ * maps dL/dN_k to dL/dN_{k+1}; record k holds its coefficients and, from the
+ * forward pass, the Stokes vector it was applied to and its length:
+ *
+ *   u    = dL/dS' = (a G a + b G b, a G a - b G b, 2 a Re G b, 2 b Im G a)
+ *   gS   = T^T u, T the step's Stokes map
+ *   G   += the transpose of the projection, at gS - u
+ *   G    = the two pushes of record k + 1, transposed
+ *
+ * Only this chain is sequential.  T comes from the coefficients and is
+ * evaluated one record per lane; u is left in the record (over its A1, read
+ * for the last time here), and k_adj_scatter, one thread per record, turns
+ * it into the gradients of the coefficients and of the fluid.  Nothing of
+ * the forward pass is recomputed.
+ *
+ * Bound by the chain of the longest ray (two pushes and four exchanges a
+ * step, ~0.7 us) and, with G = 4, by the issue rate.  A 160x160 image
+ * (25 600 rays, 3.3e7 steps): walk 97 -> 16 ms against one lane per ray with
+ * N recomputed between checkpoints and the step's derivatives in the chain,
+ * k_adj_scatter, which has them now, 7 -> 14 ms; a 40x40 image (G = 16):
+ * walk and scatter 77 -> 7 ms.  Every wait is bounded as in k_walk. */
+template <int G>
+__global__ void __launch_bounds__(32)
+    k_adj_walk(const int32_t *__restrict__ list, int n_list, double *__restrict__ pool, const int *__restrict__ next,
+               const int *__restrict__ first, const RayRec *__restrict__ rays, const double *__restrict__ dL_dout,
+               unsigned long long *__restrict__ counters, int queue)
 {
-  const DevCam &C = c_cam;
+  using W = WalkSm<G, 0>;
+  constexpr int CB = IPG_CHUNK_STEPS / G; /* blocks per chunk */
+  constexpr unsigned GM = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+  extern __shared__ __align__(16) unsigned char wsm[];
+  __shared__ __align__(8) unsigned long long wbar[W::RAYS];
+  const int lane = threadIdx.x, grp = lane / G, q = lane % G, j = lane & 3;
+  unsigned char *const slots = wsm + grp * G * W::SLOT;
+  double *const xch = reinterpret_cast<double *>(wsm + 32 * W::SLOT + grp * W::XCH);
+  unsigned long long *const bar = wbar + grp;
+  if (q == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncwarp();
   const DevGrid &Gd = c_grid;
-  constexpr int KC = K < IPG_CHUNK_STEPS ? K : IPG_CHUNK_STEPS;
-  HermN Nbuf[K];
+  const DevCam &C = c_cam;
+  unsigned ph = 0;
+  bool has = false, drained = false;
+  int n0 = 0, blk = 0, chunk = 0, cnext = -1; /* the ray's radiating records are among 0 .. n0 - 1 */
+  WalkN N;                                     /* column j of dL/dN */
+#pragma unroll
+  for (int i = 0; i < 4; i++) N.r[i] = N.s[i] = 0.;
   while (true) {
-    const unsigned long long t = atomicAdd(counter, 1ULL);
-    if (t >= (unsigned long long)n_list) return;
-    const int ray = list ? list[t] : (int)t;
-    const RayRec rec = rays[ray];
-    if (rec.status != IPG_RAY_OK) continue;
-    const int nstep = rec.nstep;
-    /* G_0 from dL/d(I, Q, U, V) of project_N (src/ipolarray.c:578-598) */
-    const double gI = dL_dout[4 * ray], gQ = dL_dout[4 * ray + 1], gU = dL_dout[4 * ray + 2],
-                 gV = dL_dout[4 * ray + 3];
-    const double gSQ = gQ * C.cproj + gU * C.sproj, gSU = -gQ * C.sproj + gU * C.cproj;
-    GradN G;
-    hn_zero(&G);
-    gn_add_stokes_adj(C.Ecov[1], C.Ecov[2], 0.5 * (gI + gSQ), 0.5 * (gI - gSQ), gSU, gV, &G);
-    ChunkWalk w = {first[ray], 0};
-    for (int lo = 0; lo < nstep; lo += K) {
-      const int hi = min(lo + K, nstep);
-      /* N_hi: zero at the source end, else the forward's checkpoint */
-      HermN N;
-      if (hi == nstep) {
-        hn_zero(&N);
-      } else {
-        walk_rec(w, hi, pool, prev, next);
-        const double *q = ckpt + (((size_t)w.chunk * IPG_CHUNK_STEPS + (hi - w.base)) / KC) * 16;
-        N.r00 = q[0]; N.r01 = q[1]; N.r02 = q[2]; N.r03 = q[3];
-        N.r11 = q[4]; N.r12 = q[5]; N.r13 = q[6]; N.r22 = q[7];
-        N.r23 = q[8]; N.r33 = q[9]; N.s01 = q[10]; N.s02 = q[11];
-        N.s03 = q[12]; N.s12 = q[13]; N.s13 = q[14]; N.s23 = q[15];
+    while (__any_sync(0xffffffffu, !has && !drained)) {
+      unsigned long long t = 0;
+      const bool want = !has && !drained;
+      if (want && q == 0) t = atomicAdd(&counters[queue], 1ULL);
+      t = __shfl_sync(0xffffffffu, t, 0, G);
+      if (!want) continue;
+      if (t >= (unsigned long long)n_list) {
+        drained = true;
+        continue;
       }
-      /* for n = hi .. lo+1, N_n after the two pushes of step n (the
-       * state evolve_N was applied to), the forward's values */
-      for (int n = hi; n > lo; n--) {
-        const double *rn = walk_rec(w, n, pool, prev, next);
-        const double *rm = walk_rec(w, n - 1, pool, prev, next);
-        HermN Np;
-        fwd_N(C, rn, rm, &N, &Np);
-        Nbuf[hi - n] = Np;
+      const int ray = list ? list[t] : (int)t;
+      const RayRec rec = rays[ray];
+      if (rec.status != IPG_RAY_OK || rec.nstep < 1) continue;
+      has = true;
+      n0 = rec.nstep;
+      blk = 0;
+      chunk = first[ray];
+      cnext = n0 > IPG_CHUNK_STEPS ? next[chunk] : -1;
+      /* G_0 from dL/d(I, Q, U, V) of project_N (src/ipolarray.c:578-598) */
+      const double gI = dL_dout[4 * ray], gQ = dL_dout[4 * ray + 1], gU = dL_dout[4 * ray + 2],
+                   gV = dL_dout[4 * ray + 3];
+      const double gSQ = gQ * C.cproj + gU * C.sproj, gSU = -gQ * C.sproj + gU * C.cproj;
+      const double *e1 = C.Ecov[1], *e2 = C.Ecov[2];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        N.r[i] = hn_upd_r(0., e1[i], e1[j], e2[i], e2[j], 0.5 * (gI + gSQ), 0.5 * (gI - gSQ), 0.5 * gSU);
+        N.s[i] = hn_upd_s(0., e1[i], e1[j], e2[i], e2[j], 0.5 * gV);
       }
-      /* the adjoint of steps n = lo+1 .. hi */
-      for (int n = lo + 1; n <= hi; n++) {
-        const double *rn = walk_rec(w, n, pool, prev, next);
-        double *rm = const_cast<double *>(walk_rec(w, n - 1, pool, prev, next));
-        const double dl = rn[REC_DL];
-        const double dlfull = dl * Gd.inv_dlfac, dlhalf = (0.5 * dl) * Gd.inv_dlfac;
-        double A1[4][4], A2[4][4];
-        load_A(rn + REC_A1, A1);
-        load_A(rn + REC_A2, A2);
-        CoefBlock cb;
-        load_coef(rm, cb);
-        const int flags = (int)cb.flags;
-        if (flags & 1) {
-          int zero_emission = (flags & 2) ? 1 : 0;
-          if (C.target_nturns >= 0 && (int)rn[REC_NTURNS] != C.target_nturns) zero_emission = 1;
-          double gc[8];
-          evolve_adj(cb, dl, zero_emission, Nbuf[hi - n], &G, gc);
-          /* dL/d(coefficients) of the record of step n-1, in place of its
-           * A1, which this walk read for the last time at step n-1;
-           * k_adj_scatter turns them into the cells' gradients */
-          store4(rm + REC_A1, gc[0], gc[1], gc[2], gc[3]);
-          store4(rm + REC_A1 + 4, gc[4], gc[5], gc[6], gc[7]);
-        }
-        /* push_polar twice, transposed: G_Nh = -dlfull (A2^T G + G A2),
-         * G_N = G + G_Nh - dlhalf (A1^T G_Nh + G_Nh A1) */
-        GradN Gh, zero;
-        hn_zero(&zero);
-        gn_push_adj(zero, G, A2, -dlfull, &Gh);
-        GradN Gs;
-        gn_push_adj(Gh, Gh, A1, -dlhalf, &Gs);
-        G.r00 += Gs.r00; G.r01 += Gs.r01; G.r02 += Gs.r02; G.r03 += Gs.r03;
-        G.r11 += Gs.r11; G.r12 += Gs.r12; G.r13 += Gs.r13; G.r22 += Gs.r22;
-        G.r23 += Gs.r23; G.r33 += Gs.r33; G.s01 += Gs.s01; G.s02 += Gs.s02;
-        G.s03 += Gs.s03; G.s12 += Gs.s12; G.s13 += Gs.s13; G.s23 += Gs.s23;
+      const int cnt = n0 < G ? n0 : G;
+      const unsigned char *src = reinterpret_cast<const unsigned char *>(step_ptr(pool, chunk, 0));
+      if (q == 0) walk_expect(bar, cnt * W::COPY);
+      if (q < cnt) walk_copy(slots + q * W::SLOT, src + (size_t)q * IPG_STEP_DOUBLES * 8, W::COPY, bar);
+    }
+    if (!__any_sync(0xffffffffu, has)) break;
+    const bool ok = !has || walk_wait(bar, ph);
+    if (__any_sync(0xffffffffu, !ok)) {
+      if (lane == 0) atomicAdd(&counters[CNT_STALL], 1ULL);
+      break;
+    }
+    if (has) ph ^= 1;
+    /* ---- one lane per record: the step's Stokes map ---- */
+    unsigned char *const my = slots + q * W::SLOT;
+    const int k = blk * G + q;
+    bool ev_my = false;
+    if (has && k < n0) {
+      const double2 *p2 = reinterpret_cast<const double2 *>(my + W::FT);
+      const double2 v0 = p2[0], v1 = p2[1], v3 = p2[3], v4 = p2[4], v5 = p2[5], v6 = p2[6];
+      ev_my = (int)v0.x & 1;
+      reinterpret_cast<double *>(my + W::FX)[8] = v1.y; /* dl of the record's pushes */
+      if (ev_my) {
+        StokesMap m;
+        stokes_map(0., 0., 0., v3.y, v4.x, v4.y, v5.y, v6.x, v6.y, &m);
+        double2 *t2 = reinterpret_cast<double2 *>(my + W::FT);
+#pragma unroll
+        for (int i = 0; i < 8; i++) t2[i] = make_double2(m.T[2 * i], m.T[2 * i + 1]);
       }
     }
+    const unsigned bal = (__ballot_sync(0xffffffffu, ev_my) >> (grp * G)) & GM;
+    /* the next block: its address and byte count */
+    const int kb = blk % CB;
+    const int cntn = has ? min(G, n0 - (blk + 1) * G) : 0; /* <= 0: none */
+    const unsigned char *src = nullptr;
+    if (cntn > 0) {
+      const int ch = kb == CB - 1 ? cnext : chunk;
+      src = reinterpret_cast<const unsigned char *>(step_ptr(pool, ch, ((kb + 1) % CB) * G));
+      if (q == 0) {
+        walk_expect(bar, cntn * W::COPY);
+        /* and the block after it, into L2 */
+        const int cnt2 = min(G, n0 - (blk + 2) * G);
+        if (CB > 1 && cnt2 > 0)
+          walk_prefetch_l2(step_ptr(pool, kb < CB - 2 ? chunk : cnext, ((kb + 2) % CB) * G), cnt2 * IPG_STEP_DOUBLES * 8);
+      }
+    }
+    /* this lane's writes of its slot come before the copies that refill it */
+    walk_refill_fence();
+    __syncwarp();
+    const int nmine = has ? min(G, n0 - blk * G) : 0;
+    const int any_n = __reduce_max_sync(0xffffffffu, nmine);
+    const unsigned any_ev = __reduce_or_sync(0xffffffffu, bal);
+    /* ---- the block's records in order ---- */
+#pragma unroll 1
+    for (int qq = 0; qq < any_n; qq++) {
+      const int kk = blk * G + qq;
+      const bool act = qq < nmine;
+      unsigned char *const sl = slots + qq * W::SLOT;
+      /* the pushes of record kk, transposed: G_h = -dl (A2^T G + G A2),
+       * G += G_h - dl/2 (A1^T G_h + G_h A1); none at record 0 */
+      if (__any_sync(0xffffffffu, act && kk >= 1)) {
+        const double dlk = reinterpret_cast<const double *>(sl + W::FX)[8];
+        const double dlfull = dlk * Gd.inv_dlfac, dlhalf = (0.5 * dlk) * Gd.inv_dlfac;
+        const double *const A1 = reinterpret_cast<const double *>(sl), *const A2 = A1 + 16;
+        double a[4][4], at[4][4];
+        WalkN Z, Gh, Gs;
+#pragma unroll
+        for (int i = 0; i < 4; i++) Z.r[i] = Z.s[i] = 0.;
+        walk_ldA(A2, a);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int l = 0; l < 4; l++) at[i][l] = a[l][i];
+        walk_push(Z, N, at, dlfull, j, xch, &Gh);
+        walk_ldA(A1, a);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int l = 0; l < 4; l++) at[i][l] = a[l][i];
+        walk_push(Gh, Gh, at, dlhalf, j, xch + 32, &Gs);
+        if (act && kk >= 1) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            N.r[i] = __dadd_rn(N.r[i], Gs.r[i]);
+            N.s[i] = __dadd_rn(N.s[i], Gs.s[i]);
+          }
+        }
+      }
+      if ((any_ev >> qq) & 1u) {
+        const bool ev = (bal >> qq) & 1u;
+        double e1[4], e2[4], a[4], b[4], g11, g22, h12, h21;
+        walk_row<0>(sl, 2, a);
+        walk_row<0>(sl, 3, b);
+        walk_row<0>(sl, 0, e1);
+        walk_row<0>(sl, 1, e2);
+        walk_stokes(N, a, b, j, &g11, &g22, &h12, &h21);
+        const double u[4] = {g11 + g22, g11 - g22, 2. * h12, 2. * h21};
+        if (ev && q == 0) store4(step_ptr(pool, chunk, kk % IPG_CHUNK_STEPS) + REC_A1, u[0], u[1], u[2], u[3]);
+        /* component j of T^T u, swapped over the lanes */
+        const double *T = reinterpret_cast<const double *>(sl + W::FT) + j;
+        const double s = dot4_rn(T[0], T[4], T[8], T[12], u[0], u[1], u[2], u[3]);
+        double gS[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) gS[i] = __shfl_sync(0xffffffffu, s, i, 4);
+        /* dL/dT: directly and through S = ((T11 + T22)/2, (T11 - T22)/2,
+         * Re T12, Im T21) */
+        const double d11 = 0.5 * (gS[0] + gS[1]) - g11, d22 = 0.5 * (gS[0] - gS[1]) - g22;
+        const double d12 = 0.5 * (gS[2] - u[2]), d21 = 0.5 * (gS[3] - u[3]);
+        const double e1j = j == 0 ? e1[0] : j == 1 ? e1[1] : j == 2 ? e1[2] : e1[3];
+        const double e2j = j == 0 ? e2[0] : j == 1 ? e2[1] : j == 2 ? e2[2] : e2[3];
+        if (ev) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            N.r[i] = hn_upd_r(N.r[i], e1[i], e1j, e2[i], e2j, d11, d22, d12);
+            N.s[i] = hn_upd_s(N.s[i], e1[i], e1j, e2[i], e2j, d21);
+          }
+        }
+      }
+      /* the slot is free: the next block's record */
+      __syncwarp();
+      if (q == qq && q < cntn) walk_copy(sl, src + (size_t)q * IPG_STEP_DOUBLES * 8, W::COPY, bar);
+    }
+    if (has) {
+      blk++;
+      if (blk * G >= n0) {
+        has = false;
+      } else if (kb == CB - 1) {
+        chunk = cnext;
+        cnext = n0 > (blk / CB + 1) * IPG_CHUNK_STEPS ? next[chunk] : -1;
+      }
+    }
+    __syncwarp();
   }
 }
 
-/* One thread per step record of the wave: the coefficient gradients the
- * walk left at each radiating record (steps 0 .. nstep-1 of a traced ray)
- * become dL/d(ne, Theta_e, |B|) at its point and are scattered to the
- * cells of its gather (fluid_scatter).  Parallel over records, where the
- * walk is one lane per ray. */
+/* One thread per step record of the wave: dL/dS' that the walk left at each
+ * radiating record (steps 0 .. nstep-1 of a traced ray) becomes the
+ * gradients of the step's coefficients (stokes_step_vjp, at the S that the
+ * forward pass left), then dL/d(ne, Theta_e, |B|) at its point, scattered to
+ * the cells of its gather (fluid_scatter). */
 __global__ void __launch_bounds__(128, 3)
     k_adj_scatter(const double *__restrict__ pool, const int2 *__restrict__ chunk_meta,
                   const unsigned long long *__restrict__ counters, long long n_chunks,
@@ -428,10 +381,19 @@ __global__ void __launch_bounds__(128, 3)
     const int s = meta.y + slot;
     if (rec.status != IPG_RAY_OK || s >= rec.nstep) continue;
     const double *p = step_ptr(const_cast<double *>(pool), c, slot);
-    if (!((int)p[REC_FLAGS] & 1)) continue;
+    const int flags = (int)p[REC_FLAGS];
+    if (!(flags & 1)) continue;
     double gc[8];
-    load4(p + REC_A1, gc);
-    load4(p + REC_A1 + 4, gc + 4);
+    {
+      const bool zero = flags & 256; /* a step without emission */
+      const double cv[8] = {zero ? 0. : p[REC_JI], zero ? 0. : p[REC_JI + 1], zero ? 0. : p[REC_JI + 2], p[REC_JI + 3],
+                            p[REC_JI + 4],         p[REC_JI + 5],             p[REC_RQ],                 p[REC_RV]};
+      const double S0[4] = {p[REC_ADJ_SI], p[REC_ADJ_SI + 1], p[REC_ADJ_SU], p[REC_ADJ_SU + 1]};
+      double u[4], gS[4];
+      load4(p + REC_A1, u);
+      stokes_step_vjp(cv, p[REC_ADJ_DL], S0, u, gS, gc);
+      if (zero) gc[0] = gc[1] = gc[2] = 0.;
+    }
     fluid_scatter(fields, adj_side + ((size_t)c * IPG_CHUNK_STEPS + slot) * IPG_ADJ_DOUBLES, C.emission_type, gc,
                   g_ne, g_th, g_b);
   }
@@ -554,9 +516,32 @@ extern "C" int ipg__check_step_vjp(int device, int n, unsigned long long seed, d
 /* ===================================================================== */
 /* host side                                                              */
 /* ===================================================================== */
-template <int K>
+/* lanes per ray as in the forward walk (walk_lanes) */
+template <int G>
+static int launch_adj_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, double *pool, const int *next,
+                             const int *first, const double *dL, unsigned long long *cnt, cudaStream_t st)
+{
+  const void *fn = (const void *)k_adj_walk<G>;
+  const size_t sm = WalkSm<G, 0>::BYTES;
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
+  k_adj_walk<G><<<wb, 32, sm, st>>>(list, (int)n, pool, next, first, ctx->d_rays, dL, cnt, CNT_N);
+  CK(cudaGetLastError());
+  return IPG_OK;
+}
+static int launch_adj_walk(ipg_ctx *ctx, const int32_t *list, size_t n, double *pool, const int *next,
+                           const int *first, const double *dL, unsigned long long *cnt, cudaStream_t st)
+{
+  switch (walk_lanes(ctx, n)) {
+    case 32: return launch_adj_walk_g<32>(ctx, list, n, pool, next, first, dL, cnt, st);
+    case 16: return launch_adj_walk_g<16>(ctx, list, n, pool, next, first, dL, cnt, st);
+    case 8: return launch_adj_walk_g<8>(ctx, list, n, pool, next, first, dL, cnt, st);
+    default: return launch_adj_walk_g<4>(ctx, list, n, pool, next, first, dL, cnt, st);
+  }
+}
+
 static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t *list, size_t run, double *pool,
-                        double *side, double *ckpt, long long n_chunks, int *next, int *first, const double *dL,
+                        double *side, long long n_chunks, int *next, int *first, const double *dL,
                         ipg_pixel_out *d_out, double *g, size_t ncell, int32_t *deferred)
 {
   const int threads = 128;
@@ -579,16 +564,14 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[3], st));
-  int rc = launch_walk<false, 0, K>(ctx, list, run, pool, ctx->d_chunk_prev, d_out, cnt, ckpt, st);
+  int rc = launch_walk<false, 0, true>(ctx, list, run, pool, ctx->d_chunk_prev, d_out, cnt, st);
   if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[4], st));
   k_adj_link<<<4 * ctx->n_sm, 256, 0, st>>>(ctx->d_chunk_prev, ctx->d_chunk_meta, cnt, n_chunks, next, first);
   CK(cudaGetLastError());
-  int ab = grid_blocks(ctx, (const void *)k_adjoint<K>, threads, run);
-  k_adjoint<K><<<ab, threads, 0, st>>>(list, (int)run, pool, side, ckpt, ctx->d_chunk_prev, next, first, ctx->d_rays,
-                                       dL, ctx->d_fields, g, g + ncell, g + 2 * ncell, cnt + CNT_N);
-  CK(cudaGetLastError());
+  rc = launch_adj_walk(ctx, list, run, pool, next, first, dL, cnt, st);
+  if (rc) return rc;
   CK(cudaEventRecord(ctx->ev_pred[0], st));
   int sb = grid_blocks(ctx, (const void *)k_adj_scatter, threads, (size_t)n_chunks * IPG_CHUNK_STEPS);
   k_adj_scatter<<<sb, threads, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays, side, ctx->d_fields, g,
@@ -629,16 +612,13 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
   CK(cudaMemcpyToSymbolAsync(c_plug, &ctx->dp, sizeof(DevPlug), 0, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyToSymbolAsync(c_cam, &dc, sizeof(DevCam), 0, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->d_ij, ij, 2 * n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  /* the pool per chunk: 32 records, their adjoint blocks, the checkpoints */
-  const int KC = K < IPG_CHUNK_STEPS ? K : IPG_CHUNK_STEPS;
+  /* the pool per chunk: 32 records and their adjoint blocks */
   const size_t rec_b = (size_t)IPG_CHUNK_STEPS * IPG_STEP_DOUBLES * sizeof(double);
   const size_t side_b = (size_t)IPG_CHUNK_STEPS * IPG_ADJ_DOUBLES * sizeof(double);
-  const size_t ck_b = (size_t)(IPG_CHUNK_STEPS / KC) * 16 * sizeof(double);
-  const long long n_chunks = (long long)(((size_t)ctx->n_chunks * rec_b) / (rec_b + side_b + ck_b));
+  const long long n_chunks = (long long)(((size_t)ctx->n_chunks * rec_b) / (rec_b + side_b));
   if (n_chunks < 16) return IPG_E_NOMEM;
   double *pool = ctx->d_pool;
   double *side = pool + (size_t)n_chunks * IPG_CHUNK_STEPS * IPG_STEP_DOUBLES;
-  double *ckpt = side + (size_t)n_chunks * IPG_CHUNK_STEPS * IPG_ADJ_DOUBLES;
   /* scratch kept in the context between calls (grow-only) */
   auto grow = [](void **ptr, size_t *cap, size_t bytes) -> cudaError_t {
     if (*cap >= bytes) return cudaSuccess;
@@ -687,12 +667,7 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     }
     CKA(cudaEventRecord(ctx->ev[0], st));
     const int em = cam->emission_type;
-    if (K == 16) rc = adjoint_wave<16>(ctx, em, ctx->d_ij, list, run, pool, side, ckpt, n_chunks, next, first, dL,
-                                       ctx->d_out, g, ncell, nextl);
-    else if (K == 32) rc = adjoint_wave<32>(ctx, em, ctx->d_ij, list, run, pool, side, ckpt, n_chunks, next, first,
-                                            dL, ctx->d_out, g, ncell, nextl);
-    else rc = adjoint_wave<64>(ctx, em, ctx->d_ij, list, run, pool, side, ckpt, n_chunks, next, first, dL,
-                               ctx->d_out, g, ncell, nextl);
+    rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, pool, side, n_chunks, next, first, dL, ctx->d_out, g, ncell, nextl);
     if (rc) return rc;
     CKA(cudaEventRecord(ctx->ev[1], st));
     unsigned long long h[CNT_N];

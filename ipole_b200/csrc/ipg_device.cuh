@@ -61,6 +61,9 @@
 #define REC_JI 36    /* jar_calc: jI jQ jV aI aQ aV (U components are zero) */
 #define REC_RQ 43    /* rho_Q, rho_V */
 #define REC_RV 44
+#define REC_ADJ_SI 33 /* the adjoint's forward pass (k_walk): S before the step that ends here, I and Q, */
+#define REC_ADJ_DL 45 /* that step's length, */
+#define REC_ADJ_SU 46 /* and S's U and V */
 #define REC_E1COV 48 /* plasma tetrad rows 1, 2: covariant, then contravariant */
 #define REC_E2COV 52
 #define REC_E1CON 56

@@ -1847,30 +1847,34 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
  * warp steps fewer rays together: the 128x128 image's longest two classes
  * (78 and 1385 rays) walk 11 ms with G = 32 and 16 against 17 ms with G = 4,
  * its bulk (14 921 rays) 5 ms with G = 4 against 12 ms with G = 32. */
-template <int G, bool S32, int RM, int CKK>
+template <int G, bool S32, int RM, bool ADJ>
 static int launch_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
-                         ipg_pixel_out *d_out, unsigned long long *cnt, double *ckpt, cudaStream_t stream)
+                         ipg_pixel_out *d_out, unsigned long long *cnt, cudaStream_t stream)
 {
-  const void *fn = (const void *)k_walk<G, S32, RM, CKK>;
+  const void *fn = (const void *)k_walk<G, S32, RM, ADJ>;
   const size_t sm = WalkSm<G, RM>::BYTES;
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
-  k_walk<G, S32, RM, CKK><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, ctx->d_rays, d_out, cnt, ckpt);
+  k_walk<G, S32, RM, ADJ><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, ctx->d_rays, d_out, cnt);
   CK(cudaGetLastError());
   return IPG_OK;
 }
 
-template <bool S32, int RM, int CKK>
-static int launch_walk(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
-                       ipg_pixel_out *d_out, unsigned long long *cnt, double *ckpt, cudaStream_t stream)
+static int walk_lanes(const ipg_ctx *ctx, size_t n)
 {
   const size_t resident = (size_t)ctx->n_sm * 8; /* warps */
-  const int G = n <= resident ? 32 : n <= 2 * resident ? 16 : n <= 4 * resident ? 8 : 4;
-  switch (G) {
-    case 32: return launch_walk_g<32, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
-    case 16: return launch_walk_g<16, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
-    case 8: return launch_walk_g<8, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
-    default: return launch_walk_g<4, S32, RM, CKK>(ctx, list, n, pool, chunk_prev, d_out, cnt, ckpt, stream);
+  return n <= resident ? 32 : n <= 2 * resident ? 16 : n <= 4 * resident ? 8 : 4;
+}
+
+template <bool S32, int RM, bool ADJ = false>
+static int launch_walk(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
+                       ipg_pixel_out *d_out, unsigned long long *cnt, cudaStream_t stream)
+{
+  switch (walk_lanes(ctx, n)) {
+    case 32: return launch_walk_g<32, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
+    case 16: return launch_walk_g<16, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
+    case 8: return launch_walk_g<8, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
+    default: return launch_walk_g<4, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
   }
 }
 
@@ -1885,7 +1889,7 @@ static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
     CK(cudaGetLastError());
     return IPG_OK;
   }
-  return launch_walk<S32, RM, 0>(ctx, b.list, b.run, b.pool, b.chunk_prev, d_out, b.cnt, nullptr, b.stream);
+  return launch_walk<S32, RM>(ctx, b.list, b.run, b.pool, b.chunk_prev, d_out, b.cnt, b.stream);
 }
 
 template <int P>

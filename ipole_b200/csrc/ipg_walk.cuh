@@ -305,14 +305,17 @@ struct WalkFac<true> {
   }
 };
 
-/* RM: record layout (0 FP64, 1 compact); CKK > 0: N before the push of every
- * record k with k % CKK == 0 is kept in ckpt, as by k_transfer */
-template <int G, bool S32, int RM, int CKK = 0>
+/* RM: record layout (0 FP64, 1 compact); ADJ (the adjoint's forward pass,
+ * FP64 records): a radiating record is left with what the adjoint reads of
+ * the step that ends there: the Stokes vector before the step, the step's
+ * length, and bit 256 of its flags where the step had no emission */
+template <int G, bool S32, int RM, bool ADJ = false>
 __global__ void __launch_bounds__(32)
     k_walk(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
            const int *__restrict__ chunk_prev, const RayRec *__restrict__ rays, ipg_pixel_out *__restrict__ out,
-           unsigned long long *__restrict__ counters, double *__restrict__ ckpt = nullptr)
+           unsigned long long *__restrict__ counters)
 {
+  static_assert(!ADJ || (RM == 0 && !S32), "the adjoint's records are FP64");
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "lanes per ray");
   using W = WalkSm<G, RM>;
   constexpr int CB = IPG_CHUNK_STEPS / G; /* blocks per chunk */
@@ -457,6 +460,11 @@ __global__ void __launch_bounds__(32)
                         reinterpret_cast<double *>(my + W::FT), reinterpret_cast<double *>(my + W::FX));
       nrad++;
       if (!unpol) flag |= flags >> 2;
+      if constexpr (ADJ) {
+        double *w = step_ptr(const_cast<double *>(pool), chunk, k % IPG_CHUNK_STEPS);
+        w[REC_FLAGS] = (double)(flags | (zero_emission ? 256 : 0));
+        w[REC_ADJ_DL] = dl_n;
+      }
     }
     /* the next block: its address, its byte count, the slots this block
      * leaves unused */
@@ -523,6 +531,14 @@ __global__ void __launch_bounds__(32)
           const double aj = j == 0 ? a[0] : j == 1 ? a[1] : j == 2 ? a[2] : a[3];
           const double bj = j == 0 ? b[0] : j == 1 ? b[1] : j == 2 ? b[2] : b[3];
           walk_stokes(N, e1, e2, j, &T11, &T22, &T12r, &T21i);
+          if constexpr (ADJ) {
+            if (ev && q == 0) {
+              double *w = step_ptr(const_cast<double *>(pool), chunk, kk % IPG_CHUNK_STEPS);
+              w[REC_ADJ_SI] = (T11 + T22) / 2;
+              w[REC_ADJ_SI + 1] = (T11 - T22) / 2;
+              *reinterpret_cast<double2 *>(w + REC_ADJ_SU) = make_double2(T12r, T21i);
+            }
+          }
           fac.apply((T11 + T22) / 2, (T11 - T22) / 2, T12r, T21i, &SI, &SQ, &SU, &SV);
           if (C.stokes_floors) stokes_floor(&SI, &SQ, &SU, &SV);
           const double d11 = (SI + SQ) - T11, d22 = (SI - SQ) - T22, dr12 = SU - T12r, di21 = SV - T21i;
@@ -533,34 +549,6 @@ __global__ void __launch_bounds__(32)
               N.s[i] = hn_upd_s(N.s[i], a[i], aj, b[i], bj, di21);
             }
             if (isnan(N.r[0]) || isnan(SI)) flag |= 4; /* lane 0's r[0] is N^00 */
-          }
-        }
-      }
-      if constexpr (CKK > 0) {
-        if (pu && kk % CKK == 0 && q < 4) {
-          constexpr int KC = CKK < IPG_CHUNK_STEPS ? CKK : IPG_CHUNK_STEPS;
-          double *p = ckpt + (((size_t)chunk * IPG_CHUNK_STEPS + kk % IPG_CHUNK_STEPS) / KC) * 16;
-          /* r00 r01 r02 r03 r11 r12 r13 r22 r23 r33, s01 s02 s03 s12 s13 s23 */
-          if (j == 0) {
-            p[0] = N.r[0];
-          } else if (j == 1) {
-            p[1] = N.r[0];
-            p[4] = N.r[1];
-            p[10] = N.s[0];
-          } else if (j == 2) {
-            p[2] = N.r[0];
-            p[5] = N.r[1];
-            p[7] = N.r[2];
-            p[11] = N.s[0];
-            p[13] = N.s[1];
-          } else {
-            p[3] = N.r[0];
-            p[6] = N.r[1];
-            p[8] = N.r[2];
-            p[9] = N.r[3];
-            p[12] = N.s[0];
-            p[14] = N.s[1];
-            p[15] = N.s[2];
           }
         }
       }

@@ -540,18 +540,16 @@ static int launch_adj_walk(ipg_ctx *ctx, const int32_t *list, size_t n, double *
   }
 }
 
-static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t *list, size_t run, double *pool,
-                        double *side, long long n_chunks, int *next, int *first, const double *dL,
+static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t *list, size_t run, bool sorted,
+                        double *pool, double *side, long long n_chunks, int *next, int *first, const double *dL,
                         ipg_pixel_out *d_out, double *g, size_t ncell, int32_t *deferred)
 {
   const int threads = 128;
   cudaStream_t st = ctx->stream;
   unsigned long long *cnt = ctx->d_cnt;
-  int gb = grid_blocks(ctx, (const void *)k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB>, threads, run);
-  k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB><<<gb, threads, 0, st>>>(d_ij, list, (int)run, pool, ctx->d_chunk_prev,
-                                                                        ctx->d_chunk_meta, n_chunks, cnt, ctx->d_rays,
-                                                                        deferred, nullptr);
-  CK(cudaGetLastError());
+  int rc = launch_geo_wave<CamOne>(ctx, 0, 0, d_ij, list, run, sorted, pool, ctx->d_chunk_prev, ctx->d_chunk_meta,
+                                   n_chunks, cnt, ctx->d_rays, deferred, nullptr, st);
+  if (rc) return rc;
   CK(cudaEventRecord(ctx->ev[2], st)); /* stage boundaries, read by ipg_adjoint */
   if (em == 1) {
     int cb = grid_blocks(ctx, (const void *)k_coeffs<IPG_PLUG_IHARM, 1, true>, threads, (size_t)n_chunks * 32);
@@ -564,7 +562,7 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[3], st));
-  int rc = launch_walk<false, 0, true>(ctx, list, run, pool, ctx->d_chunk_prev, d_out, cnt, st);
+  rc = launch_walk<false, 0, true>(ctx, list, run, pool, ctx->d_chunk_prev, d_out, cnt, st);
   if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[4], st));
@@ -667,7 +665,7 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     }
     CKA(cudaEventRecord(ctx->ev[0], st));
     const int em = cam->emission_type;
-    rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, pool, side, n_chunks, next, first, dL, ctx->d_out, g, ncell, nextl);
+    rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, list == ctx->d_sorted, pool, side, n_chunks, next, first, dL, ctx->d_out, g, ncell, nextl);
     if (rc) return rc;
     CKA(cudaEventRecord(ctx->ev[1], st));
     unsigned long long h[CNT_N];

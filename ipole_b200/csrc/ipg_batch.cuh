@@ -832,13 +832,21 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
     k_mark_pending<<<(nl + 255) / 256, 256, 0, sr>>>(it->geo_order, nl, W.rays_long);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->bev[0][2], sr));
-    int lb = grid_blocks(ctx, geo_fn, 256, R.nl);
-    if (lb > IPG_STARTED_MAX) lb = IPG_STARTED_MAX;
+    int lb;
     memset(ctx->h_started, 0, IPG_STARTED_MAX * sizeof(int));
-    k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CamTable><<<lb, 256, 0, sr>>>(
-        it->geo_ij, it->geo_order, nl, pool, ctx->d_chunk_prev, ctx->d_chunk_meta, R.cl, W.cnt_long, W.rays_long,
-        W.gdef_long, it->geo_grp, ctx->d_started);
-    CK(cudaGetLastError());
+    if (geo_coop(ctx, IPG_PLUG_IHARM, R.nl)) {
+      int rc = launch_geo_coop<CamTable>(ctx, B->unpol, B->rec_mixed, 1, it->geo_ij, it->geo_order, nl, pool,
+                                         ctx->d_chunk_prev, ctx->d_chunk_meta, R.cl, W.cnt_long, CNT_NEXT_G,
+                                         W.rays_long, W.gdef_long, it->geo_grp, sr, ctx->d_started, &lb);
+      if (rc) return rc;
+    } else {
+      lb = grid_blocks(ctx, geo_fn, 256, R.nl);
+      if (lb > IPG_STARTED_MAX) lb = IPG_STARTED_MAX;
+      k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CamTable><<<lb, 256, 0, sr>>>(
+          it->geo_ij, it->geo_order, nl, pool, ctx->d_chunk_prev, ctx->d_chunk_meta, R.cl, W.cnt_long, W.rays_long,
+          W.gdef_long, it->geo_grp, ctx->d_started);
+      CK(cudaGetLastError());
+    }
     /* the waves' blocks are launched once the class's SM-filling blocks are
      * resident (bounded host wait), so these find whole SMs */
     wait_started(ctx, lb);
@@ -901,11 +909,12 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[0], st));
-    int gb = grid_blocks(ctx, geo_fn, threads, run);
-    k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CamTable><<<gb, threads, 0, st>>>(
-        it->geo_ij, gl, (int)run, pool, ctx->d_chunk_prev, ctx->d_chunk_meta, n_chunks, W.cnt, W.rays, gnext,
-        it->geo_grp);
-    CK(cudaGetLastError());
+    /* (beside the longest class the waves keep one lane per ray: that class
+     * has the head of the list) */
+    int rc = launch_geo_wave<CamTable>(ctx, B->unpol, B->rec_mixed, it->geo_ij, gl, run,
+                                       first && !R.nl && gl && gl == it->geo_order, pool, ctx->d_chunk_prev,
+                                       ctx->d_chunk_meta, n_chunks, W.cnt, W.rays, gnext, it->geo_grp, st);
+    if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[1], st));
 #define IPG_LAUNCH_BCOEF(EMT, F, RMC)                                                                              \
   do {                                                                                                       \

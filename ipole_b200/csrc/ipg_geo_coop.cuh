@@ -305,14 +305,15 @@ __device__ __forceinline__ void gc_fetch(GeoLane &L, bool need, bool *has, bool 
                                          const int32_t *__restrict__ ij, const int32_t *__restrict__ list, int n_list,
                                          double *__restrict__ pool, int *__restrict__ chunk_prev,
                                          int2 *__restrict__ chunk_meta, long long n_chunks,
-                                         unsigned long long *__restrict__ counters, RayRec *__restrict__ rays,
-                                         int32_t *__restrict__ deferred, const int32_t *__restrict__ ray_grp)
+                                         unsigned long long *__restrict__ counters, int queue,
+                                         RayRec *__restrict__ rays, int32_t *__restrict__ deferred,
+                                         const int32_t *__restrict__ ray_grp)
 {
   while (__any_sync(0xffffffffu, need)) {
     unsigned long long t = 0, c = 0;
     int stop = 0;
     if (need && gl == 0) {
-      t = atomicAdd(&counters[CNT_NEXT_G], 1ULL);
+      t = atomicAdd(&counters[queue], 1ULL);
       if (t >= (unsigned long long)n_list) stop = 1;
       if constexpr (CS::batch) {
         /* a batch's step budget: once it is spent no further ray starts */
@@ -390,8 +391,9 @@ template <bool POL, bool MIXED, int TPB = 32, class CS = CamOne>
 __global__ void __launch_bounds__(TPB)
     k_geodesic_coop(const int32_t *__restrict__ ij, const int32_t *__restrict__ list, int n_list,
                     double *__restrict__ pool, int *__restrict__ chunk_prev, int2 *__restrict__ chunk_meta,
-                    long long n_chunks, unsigned long long *__restrict__ counters, RayRec *__restrict__ rays,
-                    int32_t *__restrict__ deferred, const int32_t *__restrict__ ray_grp, int *started = nullptr)
+                    long long n_chunks, unsigned long long *__restrict__ counters, int queue,
+                    RayRec *__restrict__ rays, int32_t *__restrict__ deferred, const int32_t *__restrict__ ray_grp,
+                    int *started = nullptr)
 {
   if (started && threadIdx.x == 0) {
     *(volatile int *)(started + blockIdx.x) = 1;
@@ -407,7 +409,7 @@ __global__ void __launch_bounds__(TPB)
   bool has = false, drained = false;
 #define GC_FETCH()                                                                                                 \
   gc_fetch<CS>(L, !has && !drained, &has, &drained, gl, ij, list, n_list, pool, chunk_prev, chunk_meta, n_chunks, \
-               counters, rays, deferred, ray_grp)
+               counters, queue, rays, deferred, ray_grp)
   GC_FETCH();
   while (__any_sync(0xffffffffu, has)) {
     const DevCam &C = CS::get(L.grp);

@@ -51,7 +51,8 @@ struct RayRec {
   int pad;
 };
 
-enum { CNT_POOL = 0, CNT_STEPS = 1, CNT_RAD = 2, CNT_DEFER = 3, CNT_NEXT_G = 4, CNT_NEXT_T = 5, CNT_STALL = 6, CNT_N = 7 };
+enum { CNT_POOL = 0, CNT_STEPS = 1, CNT_RAD = 2, CNT_DEFER = 3, CNT_NEXT_G = 4, CNT_NEXT_T = 5, CNT_STALL = 6,
+       CNT_NEXT_L = 7 /* the queue of the rays that a wave's k_geodesic_coop takes */, CNT_N = 8 };
 /* the counters of a batch wave (ipg_batch.cuh) continue the list: transfer
  * items deferred, the wave's step budget (0: none), the budget-spent flag,
  * transfer steps done */
@@ -1812,7 +1813,7 @@ static bool geo_coop(const ipg_ctx *ctx, int plug, size_t n) { return plug == IP
 template <class CS>
 static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const int32_t *d_ij, const int32_t *list,
                            size_t n, double *pool, int *chunk_prev, int2 *chunk_meta, long long n_chunks,
-                           unsigned long long *cnt, RayRec *rays, int32_t *deferred, const int32_t *grp,
+                           unsigned long long *cnt, int queue, RayRec *rays, int32_t *deferred, const int32_t *grp,
                            cudaStream_t stream, int *started, int *blocks)
 {
 #define IPG_LAUNCH_COOP(POL, MIXED, TPB)                                                                           \
@@ -1821,7 +1822,7 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
     if (started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;                                                     \
     *blocks = gb;                                                                                                  \
     k_geodesic_coop<POL, MIXED, TPB, CS><<<gb, TPB, 0, stream>>>(d_ij, list, (int)n, pool, chunk_prev, chunk_meta, \
-                                                                 n_chunks, cnt, rays, deferred, grp, started);     \
+                                                                 n_chunks, cnt, queue, rays, deferred, grp, started); \
   } while (0)
 #define IPG_LAUNCH_COOP_T(POL, MIXED)                     \
   do {                                                    \
@@ -1838,6 +1839,49 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
 #undef IPG_LAUNCH_COOP_T
 #undef IPG_LAUNCH_COOP
   CK(cudaGetLastError());
+  return IPG_OK;
+}
+
+/* The geodesics of one unsplit wave on stream st, FMKS (the adjoint's and
+ * the batches' waves).  Few rays take k_geodesic_coop, as above.  Of a larger
+ * wave sorted longest first, the head of the list takes it on a stream of its
+ * own, on SMs of its own: a wave ends on its longest rays, whose step takes
+ * 1.7 us there and 3.1 us or more with a lane per ray.  The head is an eighth
+ * of the rays, at most eight per SM (25 blocks of 48 rays: a sixth of the
+ * SMs): what follows is then under three times the mean length, which a lane
+ * per ray walks within the time of the whole wave.  Both take their records
+ * from the same pool, by the same counters; each has its own queue. */
+template <class CS>
+static int launch_geo_wave(ipg_ctx *ctx, int unpol, int mixed, const int32_t *d_ij, const int32_t *list, size_t n,
+                           bool sorted, double *pool, int *chunk_prev, int2 *chunk_meta, long long n_chunks,
+                           unsigned long long *cnt, RayRec *rays, int32_t *deferred, const int32_t *grp,
+                           cudaStream_t st)
+{
+  int blocks = 0;
+  if (geo_coop(ctx, IPG_PLUG_IHARM, n))
+    return launch_geo_coop<CS>(ctx, unpol, mixed, 0, d_ij, list, n, pool, chunk_prev, chunk_meta, n_chunks, cnt,
+                               CNT_NEXT_G, rays, deferred, grp, st, nullptr, &blocks);
+  size_t head = 0;
+  if (sorted && list && ctx->split) {
+    head = n / 8 < (size_t)ctx->n_sm * 8 ? n / 8 : (size_t)ctx->n_sm * 8;
+    cudaStream_t s2 = ctx->bstream[NB_MAX - 1];
+    /* the blocks mark their start (wait_started): nothing else may be queued
+     * before them */
+    CK(cudaStreamSynchronize(st));
+    memset(ctx->h_started, 0, IPG_STARTED_MAX * sizeof(int));
+    int rc = launch_geo_coop<CS>(ctx, unpol, mixed, 1, d_ij, list, head, pool, chunk_prev, chunk_meta, n_chunks, cnt,
+                                 CNT_NEXT_L, rays, deferred, grp, s2, ctx->d_started, &blocks);
+    if (rc) return rc;
+    CK(cudaEventRecord(ctx->ev_join[NB_MAX - 1], s2));
+    wait_started(ctx, blocks);
+  }
+  const void *fn = (const void *)k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CS>;
+  const int gb = grid_blocks(ctx, fn, 128, n - head);
+  k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CS><<<gb, 128, 0, st>>>(
+      d_ij, list ? list + head : list, (int)(n - head), pool, chunk_prev, chunk_meta, n_chunks, cnt, rays, deferred,
+      grp);
+  CK(cudaGetLastError());
+  if (head) CK(cudaStreamWaitEvent(st, ctx->ev_join[NB_MAX - 1], 0));
   return IPG_OK;
 }
 
@@ -1904,8 +1948,8 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
   CK(cudaEventRecord(b.ev[0], b.stream));
   if (geo_coop(ctx, P, b.run)) {
     int rc = launch_geo_coop<CamOne>(ctx, ctx->unpol, ctx->rec_mixed, b.split, d_ij, b.list, b.run, b.pool,
-                                     b.chunk_prev, b.chunk_meta, b.n_chunks, b.cnt, ctx->d_rays, b.deferred, nullptr,
-                                     b.stream, b.started, &b.geo_blocks);
+                                     b.chunk_prev, b.chunk_meta, b.n_chunks, b.cnt, CNT_NEXT_G, ctx->d_rays,
+                                     b.deferred, nullptr, b.stream, b.started, &b.geo_blocks);
     if (rc) return rc;
   } else {
     int gb = grid_blocks(ctx, (const void *)k_geodesic<P, 256, IPG_GEO_MINB>, gthreads, b.run);

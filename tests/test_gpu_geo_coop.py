@@ -57,3 +57,27 @@ def test_geodesic_waves_bit_identical(dumps):
             waves = c.stats()["waves"]
     assert waves > 1
     assert out[0].pol.tobytes() == out[1].pol.tobytes() and np.array_equal(out[0].nstep, out[1].nstep)
+
+
+@pytest.mark.parametrize("extra", [[], ["-unpol"], ["--target_nturns=1"]], ids=["pol", "unpol", "subring"])
+@pytest.mark.parametrize("rec", [ip.IPG_RECORDS_FP64, ip.IPG_RECORDS_MIXED])
+@pytest.mark.parametrize("n", [68, 70])
+def test_batch_wave_head_bit_identical(n, extra, rec, dumps):
+    """a batch's wave: all rays with eight lanes (68 x 68 items), or its
+    longest rays beside the others with one (70 x 70)"""
+    meta, _ = common.load_golden("c1_bright_32")
+    args = [f"--dump={dumps.get(meta)}", "--freqcgs=230e9", "--thetacam=163", "--phicam=0", "--MBH=6.5e9",
+            "--dsource=16.8e6", "--fov=160", "--trat_small=1", "--trat_large=20", f"--nx={n}", f"--ny={n}", *extra]
+    ps = [ip.Params.from_args([*args, f"--M_unit={mu}"]) for mu in (3e27, 6e27)]
+    with ip.Context(0, 8 << 30) as c:
+        models = [ip.Model.load(p) for p in ps]
+        c.set_record_precision(rec)
+        c.upload_batch(models[0])
+        imgs = c.render_batch(ps, models[0])
+        for p, m, im in zip(ps, models, imgs):
+            c.upload(m)
+            ref = c.render(p, m)
+            for k in ("unpol", "tau", "nstep"):
+                assert np.asarray(getattr(ref, k)).tobytes() == np.asarray(getattr(im, k)).tobytes(), k
+            if ref.pol is not None:
+                assert ref.pol.tobytes() == im.pol.tobytes()

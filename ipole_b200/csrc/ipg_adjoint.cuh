@@ -519,24 +519,24 @@ extern "C" int ipg__check_step_vjp(int device, int n, unsigned long long seed, d
 /* lanes per ray as in the forward walk (walk_lanes) */
 template <int G>
 static int launch_adj_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, double *pool, const int *next,
-                             const int *first, const double *dL, unsigned long long *cnt, cudaStream_t st)
+                             const int *first, const double *dL, unsigned long long *cnt, int queue, cudaStream_t st)
 {
   const void *fn = (const void *)k_adj_walk<G>;
   const size_t sm = WalkSm<G, 0>::BYTES;
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
-  k_adj_walk<G><<<wb, 32, sm, st>>>(list, (int)n, pool, next, first, ctx->d_rays, dL, cnt, CNT_N);
+  k_adj_walk<G><<<wb, 32, sm, st>>>(list, (int)n, pool, next, first, ctx->d_rays, dL, cnt, queue);
   CK(cudaGetLastError());
   return IPG_OK;
 }
 static int launch_adj_walk(ipg_ctx *ctx, const int32_t *list, size_t n, double *pool, const int *next,
-                           const int *first, const double *dL, unsigned long long *cnt, cudaStream_t st)
+                           const int *first, const double *dL, unsigned long long *cnt, int queue, cudaStream_t st)
 {
   switch (walk_lanes(ctx, n)) {
-    case 32: return launch_adj_walk_g<32>(ctx, list, n, pool, next, first, dL, cnt, st);
-    case 16: return launch_adj_walk_g<16>(ctx, list, n, pool, next, first, dL, cnt, st);
-    case 8: return launch_adj_walk_g<8>(ctx, list, n, pool, next, first, dL, cnt, st);
-    default: return launch_adj_walk_g<4>(ctx, list, n, pool, next, first, dL, cnt, st);
+    case 32: return launch_adj_walk_g<32>(ctx, list, n, pool, next, first, dL, cnt, queue, st);
+    case 16: return launch_adj_walk_g<16>(ctx, list, n, pool, next, first, dL, cnt, queue, st);
+    case 8: return launch_adj_walk_g<8>(ctx, list, n, pool, next, first, dL, cnt, queue, st);
+    default: return launch_adj_walk_g<4>(ctx, list, n, pool, next, first, dL, cnt, queue, st);
   }
 }
 
@@ -562,14 +562,26 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[3], st));
-  rc = launch_walk<false, 0, true>(ctx, list, run, pool, ctx->d_chunk_prev, d_out, cnt, st);
-  if (rc) return rc;
-  CK(cudaGetLastError());
+  /* the longest rays' walks with 32 lanes beside the others' (walk_head) */
+  const size_t head = walk_head(ctx, list, run, sorted);
+  const int32_t *tail = list ? list + head : list;
+  cudaStream_t sr = st;
+  if (head) {
+    if ((rc = walk_fork(ctx, st, &sr))) return rc;
+    rc = launch_walk<false, 0, true>(ctx, list, head, pool, ctx->d_chunk_prev, ctx->d_rays, d_out, cnt, st, CNT_NEXT_H);
+    if (rc) return rc;
+  }
+  rc = launch_walk<false, 0, true>(ctx, tail, run - head, pool, ctx->d_chunk_prev, ctx->d_rays, d_out, cnt, sr);
+  if (rc || (head && (rc = walk_join(ctx, st)))) return rc;
   CK(cudaEventRecord(ctx->ev[4], st));
   k_adj_link<<<4 * ctx->n_sm, 256, 0, st>>>(ctx->d_chunk_prev, ctx->d_chunk_meta, cnt, n_chunks, next, first);
   CK(cudaGetLastError());
-  rc = launch_adj_walk(ctx, list, run, pool, next, first, dL, cnt, st);
-  if (rc) return rc;
+  if (head) {
+    if ((rc = walk_fork(ctx, st, &sr))) return rc;
+    if ((rc = launch_adj_walk(ctx, list, head, pool, next, first, dL, cnt, CNT_N + 1, st))) return rc;
+  }
+  rc = launch_adj_walk(ctx, tail, run - head, pool, next, first, dL, cnt, CNT_N, sr);
+  if (rc || (head && (rc = walk_join(ctx, st)))) return rc;
   CK(cudaEventRecord(ctx->ev_pred[0], st));
   int sb = grid_blocks(ctx, (const void *)k_adj_scatter, threads, (size_t)n_chunks * IPG_CHUNK_STEPS);
   k_adj_scatter<<<sb, threads, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays, side, ctx->d_fields, g,
@@ -655,7 +667,7 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     size_t run = pending < wave ? pending : wave;
     size_t carry = pending - run;
     int32_t *nextl = ctx->d_list[cur ^ 1];
-    unsigned long long h0[CNT_N + 1];
+    unsigned long long h0[CNT_N + 2]; /* the wave's, and the adjoint walk's two queues */
     memset(h0, 0, sizeof(h0));
     h0[CNT_DEFER] = carry;
     CKA(cudaMemcpyAsync(ctx->d_cnt, h0, sizeof(h0), cudaMemcpyHostToDevice, st));

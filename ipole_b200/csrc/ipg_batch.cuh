@@ -22,16 +22,16 @@
  *     model, bit for bit as init_physical_quantities derives them on the
  *     host (model/iharm/model.c:610-717), and gathered like the single-image
  *     fields.
- *   - The transfer walks one lane per (instance, ray) over the shared
- *     records and the instance's coefficient block (k_xfer_batch).
+ *   - The transfer walks the (instance, ray) items over the shared records
+ *     and the instance's coefficient block: four or more lanes per item
+ *     (k_walk, BATCH) for small waves and for the longest rays of any, one
+ *     lane (k_xfer_batch) for the others of a large wave.
  *
  * Each instance's image is therefore the single-image path's image, bit for
  * bit.  Included by ipg_kernels.cu (one translation unit holds the constant
  * banks).
  */
 
-/* doubles of an instance's coefficient block: ju ku jI jQ jV aI aQ aV rQ rV */
-#define IPG_BCOEF 10
 /* instance slots of a camera group (a 32-bit mask per geodesic item) */
 #define IPG_BATCH_MAX_SLOTS 32
 static_assert(IPG_BATCH_MAX_SLOTS == IPG_BATCH_MAX_PER_CAMERA && IPG_BATCH_MAX_GROUPS == IPG_BATCH_MAX_CAMERAS,
@@ -761,11 +761,18 @@ static int batch_ws_reserve(ipg_ctx *ctx, BatchWs &w, size_t n_geo, size_t n_xf)
   return IPG_OK;
 }
 
-#define IPG_LAUNCH_XB(TPB, S32, RMC)                                                                                  \
-  do {                                                                                                          \
-    int tb = grid_blocks(ctx, (const void *)k_xfer_batch<TPB, S32, RMC>, TPB, pend_x);                               \
-    k_xfer_batch<TPB, S32, RMC><<<tb, TPB, 0, st>>>(xl, (int)pend_x, pool, side, G, ctx->d_chunk_prev, W.rays,      \
-                                                it->xf_geo, it->xf_slot, it->geo_grp, it->xf_out, W.cnt, xnext); \
+/* Transfer items per SM from which a lane walks an item (k_xfer_batch)
+ * instead of four (k_walk): with eight instances a ray, the lanes of a warp
+ * read the same records, and k_walk<4> moves each record into shared memory
+ * for each instance.  k_walk / k_xfer_batch, ms, both behind the head of the
+ * wave: 6 400 items 6.4 / 7.7, 32 768 items 13.9 / 15.7 (mixed tier 20.5 /
+ * 21.7), 80 000 items 21.4 / 16.8 (27.3 / 20.9), 204 800 items 51 / 25.5. */
+#define IPG_XB_LANE 300
+#define IPG_LAUNCH_XB(TPB, S32, RMC)                                                                                \
+  do {                                                                                                             \
+    int tb = grid_blocks(ctx, (const void *)k_xfer_batch<TPB, S32, RMC>, TPB, nt);                                 \
+    k_xfer_batch<TPB, S32, RMC><<<tb, TPB, 0, sx>>>(tail, (int)nt, pool, side, G, ctx->d_chunk_prev, W.rays,       \
+                                                    it->xf_geo, it->xf_slot, it->geo_grp, it->xf_out, W.cnt, xnext); \
   } while (0)
 
 /* Trace one level of a batch: every geodesic item once, then its step
@@ -943,26 +950,44 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
 #undef IPG_LAUNCH_BCOEF
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[2], st));
+    /* (items of the longest rays come first: xf_order follows the sorted
+     * geodesics) */
+    const WalkBatch wa = {side, G, it->xf_geo, it->xf_slot, it->geo_grp, xnext};
+    const size_t head = walk_head(ctx, xl, pend_x, first && !R.nl && xl == it->xf_order);
+    cudaStream_t sx = st;
+    if (head && (rc = walk_fork(ctx, st, &sx))) return rc;
+#define IPG_WALK_XB(S32, RMC)                                                                                        \
+  do {                                                                                                               \
+    if (head && (rc = launch_walk<S32, RMC, false, true>(ctx, xl, head, pool, ctx->d_chunk_prev, W.rays, it->xf_out, \
+                                                         W.cnt, st, CNT_NEXT_H, wa)))                                \
+      return rc;                                                                                                     \
+    const size_t nt = pend_x - head;                                                                                 \
+    const int32_t *tail = xl ? xl + head : xl;                                                                       \
+    if (nt < (size_t)ctx->n_sm * IPG_XB_LANE) {                                                                      \
+      if ((rc = launch_walk<S32, RMC, false, true>(ctx, tail, nt, pool, ctx->d_chunk_prev, W.rays, it->xf_out,       \
+                                                   W.cnt, sx, CNT_NEXT_T, wa)))                                      \
+        return rc;                                                                                                   \
+    } else if (B->xfer_threads == 256) {                                                                             \
+      IPG_LAUNCH_XB(256, S32, RMC);                                                                                  \
+    } else {                                                                                                         \
+      IPG_LAUNCH_XB(128, S32, RMC);                                                                                  \
+    }                                                                                                                \
+  } while (0)
     if (B->rec_mixed) {
-      if (B->step32) {
-        if (B->xfer_threads == 256) IPG_LAUNCH_XB(256, true, true);
-        else IPG_LAUNCH_XB(128, true, true);
-      } else {
-        if (B->xfer_threads == 256) IPG_LAUNCH_XB(256, false, true);
-        else IPG_LAUNCH_XB(128, false, true);
-      }
-    } else if (B->step32) {
-      if (B->xfer_threads == 256) IPG_LAUNCH_XB(256, true, false);
-      else IPG_LAUNCH_XB(128, true, false);
+      if (B->step32) IPG_WALK_XB(true, 1);
+      else IPG_WALK_XB(false, 1);
     } else {
-      if (B->xfer_threads == 256) IPG_LAUNCH_XB(256, false, false);
-      else IPG_LAUNCH_XB(128, false, false);
+      if (B->step32) IPG_WALK_XB(true, 0);
+      else IPG_WALK_XB(false, 0);
     }
+#undef IPG_WALK_XB
+    if (head && (rc = walk_join(ctx, st))) return rc;
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[3], st));
     unsigned long long h[CNT_NB];
     CK(cudaMemcpyAsync(h, W.cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (h[CNT_STALL]) return stall_fail(ctx);
     float a = 0.f, b = 0.f, c = 0.f;
     cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]);
     cudaEventElapsedTime(&b, ctx->ev[1], ctx->ev[2]);

@@ -61,6 +61,8 @@
 #define REC_JI 36    /* jar_calc: jI jQ jV aI aQ aV (U components are zero) */
 #define REC_RQ 43    /* rho_Q, rho_V */
 #define REC_RV 44
+/* doubles of an instance's coefficient block in a batch: ju ku jI jQ jV aI aQ aV rQ rV */
+#define IPG_BCOEF 10
 #define REC_ADJ_SI 33 /* the adjoint's forward pass (k_walk): S before the step that ends here, I and Q, */
 #define REC_ADJ_DL 45 /* that step's length, */
 #define REC_ADJ_SU 46 /* and S's U and V */

@@ -52,7 +52,9 @@ struct RayRec {
 };
 
 enum { CNT_POOL = 0, CNT_STEPS = 1, CNT_RAD = 2, CNT_DEFER = 3, CNT_NEXT_G = 4, CNT_NEXT_T = 5, CNT_STALL = 6,
-       CNT_NEXT_L = 7 /* the queue of the rays that a wave's k_geodesic_coop takes */, CNT_N = 8 };
+       CNT_NEXT_L = 7, /* the queue of the rays that a wave's k_geodesic_coop takes, */
+       CNT_NEXT_H = 8, /* and of those at the head of its walk */
+       CNT_N = 9 };
 /* the counters of a batch wave (ipg_batch.cuh) continue the list: transfer
  * items deferred, the wave's step budget (0: none), the budget-spent flag,
  * transfer steps done */
@@ -1891,15 +1893,16 @@ static int launch_geo_wave(ipg_ctx *ctx, int unpol, int mixed, const int32_t *d_
  * warp steps fewer rays together: the 128x128 image's longest two classes
  * (78 and 1385 rays) walk 11 ms with G = 32 and 16 against 17 ms with G = 4,
  * its bulk (14 921 rays) 5 ms with G = 4 against 12 ms with G = 32. */
-template <int G, bool S32, int RM, bool ADJ>
+template <int G, bool S32, int RM, bool ADJ, bool BATCH>
 static int launch_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
-                         ipg_pixel_out *d_out, unsigned long long *cnt, cudaStream_t stream)
+                         const RayRec *rays, ipg_pixel_out *d_out, unsigned long long *cnt, int queue,
+                         const WalkBatch &wa, cudaStream_t stream)
 {
-  const void *fn = (const void *)k_walk<G, S32, RM, ADJ>;
+  const void *fn = (const void *)k_walk<G, S32, RM, ADJ, BATCH>;
   const size_t sm = WalkSm<G, RM>::BYTES;
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
-  k_walk<G, S32, RM, ADJ><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, ctx->d_rays, d_out, cnt);
+  k_walk<G, S32, RM, ADJ, BATCH><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, rays, d_out, cnt, queue, wa);
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -1910,16 +1913,52 @@ static int walk_lanes(const ipg_ctx *ctx, size_t n)
   return n <= resident ? 32 : n <= 2 * resident ? 16 : n <= 4 * resident ? 8 : 4;
 }
 
-template <bool S32, int RM, bool ADJ = false>
+template <bool S32, int RM, bool ADJ = false, bool BATCH = false>
 static int launch_walk(ipg_ctx *ctx, const int32_t *list, size_t n, const double *pool, const int *chunk_prev,
-                       ipg_pixel_out *d_out, unsigned long long *cnt, cudaStream_t stream)
+                       const RayRec *rays, ipg_pixel_out *d_out, unsigned long long *cnt, cudaStream_t st,
+                       int queue = CNT_NEXT_T, const WalkBatch &wa = WalkBatch())
 {
+#define IPG_WALK_G(G) \
+  launch_walk_g<G, S32, RM, ADJ, BATCH>(ctx, list, n, pool, chunk_prev, rays, d_out, cnt, queue, wa, st)
   switch (walk_lanes(ctx, n)) {
-    case 32: return launch_walk_g<32, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
-    case 16: return launch_walk_g<16, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
-    case 8: return launch_walk_g<8, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
-    default: return launch_walk_g<4, S32, RM, ADJ>(ctx, list, n, pool, chunk_prev, d_out, cnt, stream);
+    case 32: return IPG_WALK_G(32);
+    case 16: return IPG_WALK_G(16);
+    case 8: return IPG_WALK_G(8);
+    default: return IPG_WALK_G(4);
   }
+#undef IPG_WALK_G
+}
+
+/* The head of a sorted wave's walk (the adjoint's and the batches' waves):
+ * its longest rays, which take 32 lanes each while the others share warps,
+ * so that the longest ray's walk no longer sets the wave's time; 0 where the
+ * whole wave takes 32.  An eighth of the wave, at most four rays per SM (a
+ * third of the SM's walks).  ms of the walk with a head of 0 / 1 / 2 / 4 / 8
+ * rays per SM: a 160x160 adjoint's forward walk 18.2 / 14.2 / 13.1 / 12.0 /
+ * 11.5; a batch's 6 400 items 11.5 / 9.8 / 6.9 / 6.4 / 6.4, 32 768 items 24.5
+ * / 13.6 / 13.6 / 13.9 / 13.7, 204 800 items (k_xfer_batch) 27.2 / 28.6 /
+ * 25.1 / 25.5 / 27.5. */
+static size_t walk_head(const ipg_ctx *ctx, const int32_t *list, size_t n, bool sorted)
+{
+  const int lanes = walk_lanes(ctx, n);
+  if (!sorted || !list || !ctx->split || lanes == 32) return 0;
+  const size_t most = (size_t)ctx->n_sm * 4;
+  return n / 8 < most ? n / 8 : most;
+}
+/* The head is enqueued on st itself, the rest (after fork) on a stream of
+ * its own, so that the head's blocks are placed first; join ends both. */
+static int walk_fork(ipg_ctx *ctx, cudaStream_t st, cudaStream_t *rest)
+{
+  *rest = ctx->bstream[NB_MAX - 1];
+  CK(cudaEventRecord(ctx->ev_fork, st));
+  CK(cudaStreamWaitEvent(*rest, ctx->ev_fork, 0));
+  return IPG_OK;
+}
+static int walk_join(ipg_ctx *ctx, cudaStream_t st)
+{
+  CK(cudaEventRecord(ctx->ev_join[NB_MAX - 1], ctx->bstream[NB_MAX - 1]));
+  CK(cudaStreamWaitEvent(st, ctx->ev_join[NB_MAX - 1], 0));
+  return IPG_OK;
 }
 
 template <bool S32, int RM>
@@ -1933,7 +1972,7 @@ static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
     CK(cudaGetLastError());
     return IPG_OK;
   }
-  return launch_walk<S32, RM>(ctx, b.list, b.run, b.pool, b.chunk_prev, d_out, b.cnt, b.stream);
+  return launch_walk<S32, RM>(ctx, b.list, b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt, b.stream);
 }
 
 template <int P>

@@ -309,15 +309,28 @@ struct WalkFac<true> {
  * FP64 records): a radiating record is left with what the adjoint reads of
  * the step that ends there: the Stokes vector before the step, the step's
  * length, and bit 256 of its flags where the step had no emission */
-template <int G, bool S32, int RM, bool ADJ = false>
+/* BATCH: the items of a batch wave.  Item t of the list is instance slot
+ * xf_slot[t] of the trajectory xf_geo[t]; its coefficients come from the
+ * instance's blocks of the side pool (IPG_BCOEF doubles per record, by a
+ * second bulk copy into the factors' area, which is written once they are
+ * read), the rest from the record that the instances share. */
+struct WalkBatch {
+  const double *side;
+  int slots; /* instance slots per camera group */
+  const int32_t *xf_geo, *xf_slot, *geo_grp;
+  int32_t *deferred;
+};
+template <int G, bool S32, int RM, bool ADJ = false, bool BATCH = false>
 __global__ void __launch_bounds__(32)
     k_walk(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
            const int *__restrict__ chunk_prev, const RayRec *__restrict__ rays, ipg_pixel_out *__restrict__ out,
-           unsigned long long *__restrict__ counters)
+           unsigned long long *__restrict__ counters, int queue, const WalkBatch B = WalkBatch())
 {
   static_assert(!ADJ || (RM == 0 && !S32), "the adjoint's records are FP64");
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "lanes per ray");
   using W = WalkSm<G, RM>;
+  constexpr unsigned BYTES = W::COPY + (BATCH ? IPG_BCOEF * 8 : 0); /* copied per record */
+  static_assert(W::COPY + IPG_BCOEF * 8 <= W::SLOT, "the coefficient block fits the factors' area");
   constexpr int CB = IPG_CHUNK_STEPS / G; /* blocks per chunk */
   constexpr unsigned GM = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
   extern __shared__ __align__(16) unsigned char wsm[];
@@ -330,8 +343,15 @@ __global__ void __launch_bounds__(32)
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncwarp();
   const DevGrid &Gd = c_grid;
-  const DevCam &C = c_cam;
-  const int unpol = C.unpol;
+  const int unpol = BATCH ? c_cams[0].unpol : c_cam.unpol; /* a batch's instances share it */
+  int cam = 0, kslot = 0;
+  /* record r (0 .. 31) of chunk ch into slot sl of the ray */
+  auto copy = [&](int sl, int ch, int r) {
+    walk_copy(slots + sl * W::SLOT, step_ptr(const_cast<double *>(pool), ch, r), W::COPY, bar);
+    if constexpr (BATCH)
+      walk_copy(slots + sl * W::SLOT + W::FX, B.side + (((size_t)ch * IPG_CHUNK_STEPS + r) * B.slots + kslot) * IPG_BCOEF,
+                IPG_BCOEF * 8, bar);
+  };
   unsigned ph = 0;
   bool has = false, drained = false;
   int ray = 0, n0 = 0, blk = 0, chunk = 0, cprev = -1, flag = 0;
@@ -348,7 +368,20 @@ __global__ void __launch_bounds__(32)
     while (__any_sync(0xffffffffu, !has && !drained)) {
       unsigned long long t = 0;
       const bool want = !has && !drained;
-      if (want && q == 0) t = atomicAdd(&counters[CNT_NEXT_T], 1ULL);
+      if (want && q == 0) {
+        bool stop = false;
+        if constexpr (BATCH) {
+          /* the batch's step budget: once it is spent no further item starts */
+          const unsigned long long budget = counters[CNT_BUDGET];
+          if (budget && *(volatile unsigned long long *)&counters[CNT_XSTEPS] +
+                                *(volatile unsigned long long *)&counters[CNT_STEPS] >=
+                            budget) {
+            counters[CNT_TIMEOUT] = 1;
+            stop = true;
+          }
+        }
+        t = stop ? ~0ULL : atomicAdd(&counters[queue], 1ULL);
+      }
       t = __shfl_sync(0xffffffffu, t, 0, G);
       if (!want) continue;
       if (t >= (unsigned long long)n_list) {
@@ -356,8 +389,13 @@ __global__ void __launch_bounds__(32)
         continue;
       }
       ray = list ? list[t] : (int)t;
-      const RayRec rec = rays[ray];
-      if (rec.status == IPG_RAY_POOL_FULL) continue;
+      const int geo = BATCH ? B.xf_geo[ray] : ray;
+      const RayRec rec = rays[geo];
+      if (rec.status == IPG_RAY_POOL_FULL) {
+        if constexpr (BATCH)
+          if (q == 0) B.deferred[atomicAdd(&counters[CNT_XDEFER], 1ULL)] = ray;
+        continue;
+      }
       if (rec.status == IPG_RAY_MAXNSTEP) {
         if (q == 0) {
           ipg_pixel_out o;
@@ -369,6 +407,10 @@ __global__ void __launch_bounds__(32)
         continue;
       }
       has = true;
+      if constexpr (BATCH) {
+        cam = B.geo_grp[geo];
+        kslot = B.xf_slot[ray];
+      }
       n0 = rec.nstep;
       blk = n0 / G;
       chunk = rec.last_chunk;
@@ -380,10 +422,8 @@ __global__ void __launch_bounds__(32)
       /* the top block's records (the slots are free: the last ray's steps
        * are done, and its reads ordered by the warp's barriers) */
       const int cnt = n0 - blk * G + 1;
-      const unsigned char *src =
-          reinterpret_cast<const unsigned char *>(step_ptr(const_cast<double *>(pool), chunk, (blk % CB) * G));
-      if (q == 0) walk_expect(bar, cnt * W::COPY);
-      if (q < cnt) walk_copy(slots + q * W::SLOT, src + (size_t)q * IPG_STEP_DOUBLES * 8, W::COPY, bar);
+      if (q == 0) walk_expect(bar, cnt * BYTES);
+      if (q < cnt) copy(q, chunk, (blk % CB) * G + q);
     }
     if (!__any_sync(0xffffffffu, has)) break;
     const bool ok = !has || walk_wait(bar, ph);
@@ -395,6 +435,7 @@ __global__ void __launch_bounds__(32)
       break;
     }
     if (has) ph ^= 1;
+    const DevCam &C = BATCH ? c_cams[cam] : c_cam;
     /* ---- phase A: one lane per record ---- */
     unsigned char *const my = slots + q * W::SLOT;
     const int k = blk * G + q;
@@ -410,18 +451,38 @@ __global__ void __launch_bounds__(32)
 #pragma unroll
       for (int i = 0; i < 7; i++) v[i] = p2[i];
       flags = (int)v[0].x;
+      dl = v[1].y;
+      nt = v[5].x;
+      if constexpr (BATCH) {
+        /* (left unwritten at records that do not radiate, and unused there) */
+        const double2 *b2 = reinterpret_cast<const double2 *>(my + W::FX);
+        v[6] = b2[4];
+        v[5] = b2[4];
+        v[4] = b2[3];
+        v[3] = b2[2];
+        v[2] = b2[1];
+        ju = b2[0].x;
+        ku = b2[0].y;
+        c[0] = v[2].x; /* jI jQ jV aI aQ aV rQ rV */
+        c[1] = v[2].y;
+        c[2] = v[3].x;
+        c[3] = v[3].y;
+        c[4] = v[4].x;
+        c[5] = v[4].y;
+        c[6] = v[5].x;
+        c[7] = v[5].y;
+      } else {
       ju = v[0].y;
       ku = v[1].x;
-      dl = v[1].y;
-      c[0] = v[2].x; /* jI jQ jV aI aQ aV rQ rV */
+      c[0] = v[2].x;
       c[1] = v[2].y;
       c[2] = v[3].x;
       c[3] = v[3].y;
       c[4] = v[4].x;
       c[5] = v[4].y;
-      nt = v[5].x;
       c[6] = v[5].y;
       c[7] = v[6].x;
+      }
     }
     const bool ev_my = valid && k < n0 && (flags & 1);
     const unsigned bal = (__ballot_sync(0xffffffffu, ev_my) >> (grp * G)) & GM;
@@ -469,14 +530,11 @@ __global__ void __launch_bounds__(32)
     /* the next block: its address, its byte count, the slots this block
      * leaves unused */
     const bool more = has && blk > 0;
-    const unsigned char *src = nullptr;
     const int kb = blk % CB;
+    const int ch = kb ? chunk : cprev, r0 = (kb ? kb - 1 : CB - 1) * G;
     if (more) {
-      const int ch = kb ? chunk : cprev;
-      src = reinterpret_cast<const unsigned char *>(
-          step_ptr(const_cast<double *>(pool), ch, (kb ? kb - 1 : CB - 1) * G));
       if (q == 0) {
-        walk_expect(bar, G * W::COPY);
+        walk_expect(bar, G * BYTES);
         /* and the block after it, into L2 */
         if (CB > 1 && blk > 1 && (kb != 1 || cprev >= 0)) {
           const int ch2 = kb == 1 ? cprev : ch;
@@ -488,9 +546,7 @@ __global__ void __launch_bounds__(32)
     /* this lane's writes of its slot come before the copies that refill it */
     walk_refill_fence();
     __syncwarp();
-    if (more && k > n0) {
-      walk_copy(my, src + (size_t)q * IPG_STEP_DOUBLES * 8, W::COPY, bar);
-    }
+    if (more && k > n0) copy(q, ch, r0 + q);
     /* which of the block's steps any ray of the warp has: records walked,
      * radiating steps, pushes */
     const unsigned mine = has ? (n0 - blk * G >= G - 1 ? GM : (2u << (n0 - blk * G)) - 1u) : 0u;
@@ -569,7 +625,7 @@ __global__ void __launch_bounds__(32)
       /* the slot is free: the next block's record (the copy's writes follow
        * this warp's reads; its writes of the factors were fenced above) */
       __syncwarp();
-      if (more && act && q == qq) walk_copy(sl, src + (size_t)q * IPG_STEP_DOUBLES * 8, W::COPY, bar);
+      if (more && act && q == qq) copy(q, ch, r0 + q);
     }
     /* the end of a ray: project_N in the camera's tetrad */
     const bool fin = has && blk == 0;
@@ -588,6 +644,7 @@ __global__ void __launch_bounds__(32)
         if (!unpol && (tauF > 1.e100 || tauF < -1.e100 || isnan(tauF))) fl |= 2;
         xfer_output(C, I, tau, tauF, T11, T22, T12r, T21i, unpol, n0, fl, &o);
         out[ray] = o;
+        if constexpr (BATCH) atomicAdd(&counters[CNT_XSTEPS], (unsigned long long)n0);
       }
       if (fin) has = false;
       __syncwarp();

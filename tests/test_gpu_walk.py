@@ -67,3 +67,28 @@ def test_walk_options_bit_identical(extra, dumps):
     for rec, step in FORMS:
         a, b = _trace(m, cam, ij, "0", rec, step), _trace(m, cam, ij, None, rec, step)
         assert a.tobytes() == b.tobytes(), (extra, rec, step)
+
+
+@pytest.mark.parametrize("n,extra", [(3, []), (25, ["--target_nturns=1"]), (40, ["--stokes_floors=1"]), (50, ["-unpol"]),
+                                     (50, [])])
+def test_batch_walk_bit_identical(n, extra, dumps):
+    """the batches' walk (the instances' coefficients from their own blocks)
+    with 32, 16, 8 and 4 lanes per item against each instance's own render,
+    in every form"""
+    meta, _ = common.load_golden("c1_bright_32")
+    args = [f"--dump={dumps.get(meta)}", "--freqcgs=230e9", "--thetacam=163", "--phicam=0", "--MBH=6.5e9",
+            "--dsource=16.8e6", "--fov=160", "--trat_small=1", "--trat_large=20", f"--nx={n}", f"--ny={n}", *extra]
+    ps = [ip.Params.from_args([*args, f"--M_unit={mu}"]) for mu in (3e27, 6e27)]
+    models = [ip.Model.load(p) for p in ps]
+    for rec, step in FORMS:
+        with ip.Context(0, 4 << 30) as c:
+            c.set_record_precision(rec)
+            c.set_step_precision(step)
+            c.upload_batch(models[0])
+            imgs = c.render_batch(ps, models[0])
+            for p, m, im in zip(ps, models, imgs):
+                c.upload(m)
+                ref = c.render(p, m)
+                for k in ("unpol", "tau", "nstep", "pol"):
+                    a, b = getattr(ref, k), getattr(im, k)
+                    assert (a is None) == (b is None) and (a is None or a.tobytes() == b.tobytes()), (n, rec, step, k)

@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(32)
   extern __shared__ __align__(16) unsigned char wsm[];
   __shared__ __align__(8) unsigned long long wbar[W::RAYS];
   const int lane = threadIdx.x, grp = lane / G, q = lane % G, j = lane & 3;
-  unsigned char *const slots = wsm + grp * G * W::SLOT;
-  double *const xch = reinterpret_cast<double *>(wsm + 32 * W::SLOT + grp * W::XCH);
+  unsigned char *const slots = wsm + grp * W::RAY;
+  double *const xch = reinterpret_cast<double *>(wsm + W::RAYS * W::RAY + grp * W::XCH);
   unsigned long long *const bar = wbar + grp;
   if (q == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -73,10 +73,15 @@ __device__ __forceinline__ void walk_prefetch_l2(const void *src, unsigned bytes
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-/* Shared memory of a warp: 32 record slots (the record, its factors over
- * the coefficients once these are read, and the extra factors behind it),
- * then the exchange areas of its rays.  Strides are odd multiples of 16
- * bytes, so that a quarter-warp's 16-byte accesses hit distinct banks; the
+/* Shared memory of a warp: per ray G record slots (the record, its factors
+ * over the coefficients once these are read, and the extra factors behind
+ * it), then the exchange areas of the rays.  Phase A reads one slot per lane,
+ * phase B one slot per ray, both in 16-byte accesses of which a quarter-warp
+ * and a ray each should hit banks of their own: in units of 16 bytes modulo 8
+ * the rays' stride is odd, and the slots' stride odd, or even but not a
+ * multiple of 4 where a quarter-warp holds two rays (G = 4).  (With one stride
+ * for both, eight rays' reads fell into a quarter of the banks, a 5-way
+ * conflict; a 160x160 image's 25 600 rays: 12.0 ms then, 10.8 now.)  The
  * exchange stride is 32 modulo 128, so that four rays' 32-byte rows do. */
 template <int G, int RM>
 struct WalkSm {
@@ -84,10 +89,11 @@ struct WalkSm {
   static constexpr int COPY = RM ? 320 : 512;
   static constexpr int FT = RM ? RECM_COEF * 8 : REC_FLAGS * 8; /* the coefficient block's 128 bytes */
   static constexpr int FX = COPY;                               /* 10 doubles: u, p, q, dtau, dtauF, dl, - */
-  static constexpr int SLOT = COPY + 80;
+  static constexpr int SLOT = COPY + (G == 4 ? 96 : 80);
+  static constexpr int RAY = G * SLOT + 16;
   static constexpr int XCH = 544; /* A N of the half and of the full push (256 each) */
-  static constexpr int BYTES = 32 * SLOT + RAYS * XCH;
-  static_assert(SLOT % 32 == 16 && XCH % 128 == 32, "bank layout");
+  static constexpr int BYTES = RAYS * (RAY + XCH);
+  static_assert((G == 4 ? SLOT % 64 == 32 : SLOT % 32 == 16) && RAY % 32 == 16 && XCH % 128 == 32, "bank layout");
 };
 
 /* Column j of N: R[.][j] and S[.][j] (S[j][j] = 0) */
@@ -336,8 +342,8 @@ __global__ void __launch_bounds__(32)
   extern __shared__ __align__(16) unsigned char wsm[];
   __shared__ __align__(8) unsigned long long wbar[W::RAYS];
   const int lane = threadIdx.x, grp = lane / G, q = lane % G, j = lane & 3;
-  unsigned char *const slots = wsm + grp * G * W::SLOT;
-  double *const xch = reinterpret_cast<double *>(wsm + 32 * W::SLOT + grp * W::XCH);
+  unsigned char *const slots = wsm + grp * W::RAY;
+  double *const xch = reinterpret_cast<double *>(wsm + W::RAYS * W::RAY + grp * W::XCH);
   unsigned long long *const bar = wbar + grp;
   if (q == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -362,7 +362,10 @@ __global__ void __launch_bounds__(32)
  * gradients of the step's coefficients (stokes_step_vjp, at the S that the
  * forward pass left), then dL/d(ne, Theta_e, |B|) at its point, scattered to
  * the cells of its gather (fluid_scatter). */
-__global__ void __launch_bounds__(128, 3)
+#ifndef IPG_SCAT_TPB
+#define IPG_SCAT_TPB 384 /* one block per SM at 168 registers */
+#endif
+__global__ void __launch_bounds__(IPG_SCAT_TPB, 1)
     k_adj_scatter(const double *__restrict__ pool, const int2 *__restrict__ chunk_meta,
                   const unsigned long long *__restrict__ counters, long long n_chunks,
                   const RayRec *__restrict__ rays, const double *__restrict__ adj_side,
@@ -373,8 +376,10 @@ __global__ void __launch_bounds__(128, 3)
   long long used = (long long)counters[CNT_POOL];
   if (used > n_chunks) used = n_chunks;
   const long long total = used * IPG_CHUNK_STEPS;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
+  for (long long t0 = blockIdx.x * (long long)blockDim.x; t0 < total; t0 += (long long)gridDim.x * blockDim.x) {
+    __syncthreads(); /* the warps share their instruction fetches, as in k_coeffs */
+    const long long t = t0 + threadIdx.x;
+    if (t >= total) continue;
     const int c = (int)(t / IPG_CHUNK_STEPS), slot = (int)(t % IPG_CHUNK_STEPS);
     const int2 meta = chunk_meta[c];
     const RayRec rec = rays[meta.x];
@@ -544,7 +549,6 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
                         double *pool, double *side, long long n_chunks, int *next, int *first, const double *dL,
                         ipg_pixel_out *d_out, double *g, size_t ncell, int32_t *deferred)
 {
-  const int threads = 128;
   cudaStream_t st = ctx->stream;
   unsigned long long *cnt = ctx->d_cnt;
   int rc = launch_geo_wave<CamOne>(ctx, 0, 0, d_ij, list, run, sorted, pool, ctx->d_chunk_prev, ctx->d_chunk_meta,
@@ -552,12 +556,12 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   if (rc) return rc;
   CK(cudaEventRecord(ctx->ev[2], st)); /* stage boundaries, read by ipg_adjoint */
   if (em == 1) {
-    int cb = grid_blocks(ctx, (const void *)k_coeffs<IPG_PLUG_IHARM, 1, true>, threads, (size_t)n_chunks * 32);
-    k_coeffs<IPG_PLUG_IHARM, 1, true><<<cb, threads, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays,
+    int cb = grid_blocks(ctx, (const void *)k_coeffs<IPG_PLUG_IHARM, 1, true>, IPG_COEF_TPB, (size_t)n_chunks * 32);
+    k_coeffs<IPG_PLUG_IHARM, 1, true><<<cb, IPG_COEF_TPB, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays,
                                                               ctx->d_fields, side);
   } else {
-    int cb = grid_blocks(ctx, (const void *)k_coeffs<IPG_PLUG_IHARM, 4, true>, threads, (size_t)n_chunks * 32);
-    k_coeffs<IPG_PLUG_IHARM, 4, true><<<cb, threads, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays,
+    int cb = grid_blocks(ctx, (const void *)k_coeffs<IPG_PLUG_IHARM, 4, true>, IPG_COEF_TPB, (size_t)n_chunks * 32);
+    k_coeffs<IPG_PLUG_IHARM, 4, true><<<cb, IPG_COEF_TPB, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays,
                                                               ctx->d_fields, side);
   }
   CK(cudaGetLastError());
@@ -583,8 +587,8 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   rc = launch_adj_walk(ctx, tail, run - head, pool, next, first, dL, cnt, CNT_N, sr);
   if (rc || (head && (rc = walk_join(ctx, st)))) return rc;
   CK(cudaEventRecord(ctx->ev_pred[0], st));
-  int sb = grid_blocks(ctx, (const void *)k_adj_scatter, threads, (size_t)n_chunks * IPG_CHUNK_STEPS);
-  k_adj_scatter<<<sb, threads, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays, side, ctx->d_fields, g,
+  int sb = grid_blocks(ctx, (const void *)k_adj_scatter, IPG_SCAT_TPB, (size_t)n_chunks * IPG_CHUNK_STEPS);
+  k_adj_scatter<<<sb, IPG_SCAT_TPB, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays, side, ctx->d_fields, g,
                                         g + ncell, g + 2 * ncell);
   CK(cudaGetLastError());
   return IPG_OK;

@@ -166,11 +166,8 @@ __device__ __forceinline__ void store_shared_m(double *p, int flags, double dl, 
   t[3] = make_float4((float)b[0], (float)b[1], (float)b[2], (float)b[3]);
 }
 
-#ifndef IPG_BCOEF_MINB
-#define IPG_BCOEF_MINB IPG_COEF_MINB /* blocks of 128 per SM the batch's coefficient pass is compiled for */
-#endif
 template <int EM, bool F32 = false, bool RM = false>
-__global__ void __launch_bounds__(128, IPG_BCOEF_MINB)
+__global__ void __launch_bounds__(IPG_COEF_TPB, IPG_COEF_MINB)
     k_coef_batch(double *__restrict__ pool, double *__restrict__ side, int G, const int2 *__restrict__ chunk_meta,
                  const unsigned long long *__restrict__ counters, long long n_chunks, const RayRec *__restrict__ rays,
                  const int32_t *__restrict__ geo_grp, const uint32_t *__restrict__ geo_mask,
@@ -181,8 +178,11 @@ __global__ void __launch_bounds__(128, IPG_BCOEF_MINB)
   long long used = (long long)counters[CNT_POOL];
   if (used > n_chunks) used = n_chunks;
   const long long total = used * IPG_CHUNK_STEPS;
-  for (long long t = c_first * IPG_CHUNK_STEPS + blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
+  for (long long t0 = c_first * IPG_CHUNK_STEPS + blockIdx.x * (long long)blockDim.x; t0 < total;
+       t0 += (long long)gridDim.x * blockDim.x) {
+    __syncthreads(); /* the warps share their instruction fetches, as in k_coeffs */
+    const long long t = t0 + threadIdx.x;
+    if (t >= total) continue;
     int c = (int)(t / IPG_CHUNK_STEPS), slot = (int)(t % IPG_CHUNK_STEPS);
     int2 meta = chunk_meta[c];
     if (meta.x < 0) continue;
@@ -925,8 +925,8 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
     CK(cudaEventRecord(ctx->ev[1], st));
 #define IPG_LAUNCH_BCOEF(EMT, F, RMC)                                                                              \
   do {                                                                                                       \
-    int cb = grid_blocks(ctx, (const void *)k_coef_batch<EMT, F, RMC>, threads, (size_t)n_chunks * IPG_CHUNK_STEPS); \
-    k_coef_batch<EMT, F, RMC><<<cb, threads, 0, st>>>(pool, side, G, ctx->d_chunk_meta, W.cnt, n_chunks, W.rays,  \
+    int cb = grid_blocks(ctx, (const void *)k_coef_batch<EMT, F, RMC>, IPG_COEF_TPB, (size_t)n_chunks * IPG_CHUNK_STEPS); \
+    k_coef_batch<EMT, F, RMC><<<cb, IPG_COEF_TPB, 0, st>>>(pool, side, G, ctx->d_chunk_meta, W.cnt, n_chunks, W.rays,  \
                                                  it->geo_grp, it->geo_mask, B->m.fourv, B->m.sets,          \
                                                  (long long)B->m.ncell, c_first);                             \
   } while (0)

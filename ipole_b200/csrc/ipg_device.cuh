@@ -75,17 +75,18 @@
  * kernels (register budget) and whether the large device functions are
  * kept out of line (smaller code, fewer instruction-cache misses).
  * k_coeffs is fully parallel, so it trades a few spilled registers for
- * occupancy: 4 blocks of 128 threads (128 registers) measured 104 ms against
- * 144 ms at 2 blocks (254 registers) on a 400x400 image; the sequential
- * kernels measured best without a cap. */
+ * occupancy: 512 threads per SM (128 registers) measured 104 ms against 144
+ * ms with 256 (254 registers) on a 400x400 image; the sequential kernels
+ * measured best without a cap. */
 #ifndef IPG_GEO_MINB
 #define IPG_GEO_MINB 1
 #endif
 #ifndef IPG_XFER_MINB
 #define IPG_XFER_MINB 1
 #endif
+#define IPG_COEF_TPB 256 /* threads per block of the coefficient passes */
 #ifndef IPG_COEF_MINB
-#define IPG_COEF_MINB 4
+#define IPG_COEF_MINB 2
 #endif
 #ifdef IPG_NOINLINE_HEAVY
 #define IPG_HEAVY __device__ __noinline__
@@ -714,22 +715,11 @@ __device__ __forceinline__ void hn_update(HermN *N, const double a[4], const dou
 /* --------------------------------------------------------------------- */
 #include "ipg_bessel_coeffs.h"
 
-/* Rolled loops keep the code of k_coeffs small (its straight-line code
- * otherwise outgrows the instruction cache). */
-#ifndef IPG_ROLL_POLY
-#define IPG_ROLL_POLY 1
-#endif
-#if IPG_ROLL_POLY
-#define IPG_POLY_LOOP _Pragma("unroll 1")
-#else
-#define IPG_POLY_LOOP _Pragma("unroll")
-#endif
-
 template <int N>
 __device__ __forceinline__ double horner(const double (&c)[N], double y)
 {
   double r = c[N - 1];
-  IPG_POLY_LOOP
+#pragma unroll
   for (int k = N - 2; k >= 0; k--) r = fma(r, y, c[k]);
   return r;
 }
@@ -738,7 +728,7 @@ template <int N>
 __device__ __forceinline__ double clenshaw(const double (&c)[N], double s)
 {
   double b1 = 0., b2 = 0., s2 = 2. * s;
-  IPG_POLY_LOOP
+#pragma unroll
   for (int k = N - 1; k >= 1; k--) {
     double t = fma(s2, b1, c[k] - b2);
     b2 = b1;

@@ -30,7 +30,7 @@ template <int N>
 __device__ __forceinline__ float hornerf(const double (&c)[N], float y)
 {
   float r = (float)c[N - 1];
-  IPG_POLY_LOOP
+#pragma unroll
   for (int k = N - 2; k >= 0; k--) r = fmaf(r, y, (float)c[k]);
   return r;
 }
@@ -39,7 +39,7 @@ template <int N>
 __device__ __forceinline__ float clenshawf(const double (&c)[N], float s)
 {
   float b1 = 0.f, b2 = 0.f, s2 = 2.f * s;
-  IPG_POLY_LOOP
+#pragma unroll
   for (int k = N - 1; k >= 1; k--) {
     float t = fmaf(s2, b1, (float)c[k] - b2);
     b2 = b1;

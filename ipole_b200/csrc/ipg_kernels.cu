@@ -592,6 +592,17 @@ __global__ void __launch_bounds__(128, IPG_GEO_MINB)
 /* ===================================================================== */
 /* k_coeffs                                                               */
 /* ===================================================================== */
+/* A block's warps start each record together (a barrier per record): the
+ * straight-line code of a record, ~90 KB, is larger than the instruction
+ * cache, and warps that drift apart each wait for its lines (no_instruction
+ * was the largest stall, 3.3 of 12.4 cycles per issue; with the barrier
+ * below 0.4).  Blocks of 256: with 128 fewer warps share a fetch, with 512
+ * two blocks no longer cover each other's barriers.  With it the Bessel
+ * polynomials are unrolled: a rolled loop waits for each coefficient's
+ * constant load.  A 160x160 image's pass 10.3 -> 8.3 ms; 400x400
+ * images (against other builds on the same box) 169 -> 163-167 ms, mixed tier
+ * 151 -> 132 ms.  Bound now by its gathers and by 8-cycle FP64 dependencies
+ * at four warps per scheduler (128 registers). */
 /* One thread per stored step s of a finished ray: everything the transfer
  * step ending at s needs that does not depend on the radiation field.  The
  * record's geodesic block is overwritten by the coefficient block; dl and
@@ -604,7 +615,7 @@ __global__ void __launch_bounds__(128, IPG_GEO_MINB)
  * (jar_both_f32). */
 #define IPG_ADJ_DOUBLES 8
 template <int P, int EM = 0, bool ADJ = false, bool F32 = false>
-__global__ void __launch_bounds__(128, IPG_COEF_MINB)
+__global__ void __launch_bounds__(IPG_COEF_TPB, IPG_COEF_MINB)
     k_coeffs(double *__restrict__ pool, const int2 *__restrict__ chunk_meta,
              const unsigned long long *__restrict__ counters, long long n_chunks,
              const RayRec *__restrict__ rays, const double *__restrict__ fields, double *__restrict__ adj_side)
@@ -615,60 +626,72 @@ __global__ void __launch_bounds__(128, IPG_COEF_MINB)
   long long used = (long long)counters[CNT_POOL];
   if (used > n_chunks) used = n_chunks;
   const long long total = used * IPG_CHUNK_STEPS;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    int c = (int)(t / IPG_CHUNK_STEPS), slot = (int)(t % IPG_CHUNK_STEPS);
-    int2 meta = chunk_meta[c];
-    RayRec rec = rays[meta.x];
-    int s = meta.y + slot;
-    if (rec.status != IPG_RAY_OK || s > rec.nstep) continue;
-    double *p = step_ptr(pool, c, slot);
-    double X1 = p[REC_X1], X2 = p[REC_X2], X3 = p[REC_X3];
-    double K[4];
-    load4(p + REC_K, K);
-    PointGeo pg;
-    point_geo<PlugT<P>::MET>(X1, X2, &pg);
-    int flags = radiating_t<P>(pg) ? 1 : 0;
-    /* isolate_counterjet, src/ipolarray.c:128-136 */
-    if (C.counterjet == 1) {
-      if (X2 < (G.cstopx[2] - G.cstartx[2]) / 2) flags |= 2;
-    } else if (C.counterjet == 2) {
-      if (X2 > (G.cstopx[2] - G.cstartx[2]) / 2) flags |= 2;
+  for (long long t0 = blockIdx.x * (long long)blockDim.x; t0 < total; t0 += (long long)gridDim.x * blockDim.x) {
+    __syncthreads();
+    const long long t = t0 + threadIdx.x;
+    const int c = (int)(t / IPG_CHUNK_STEPS), slot = (int)(t % IPG_CHUNK_STEPS);
+    double *p = nullptr;
+    bool live = t < total, end = false;
+    if (live) {
+      const int2 meta = chunk_meta[c];
+      const RayRec rec = rays[meta.x];
+      const int s = meta.y + slot;
+      live = rec.status == IPG_RAY_OK && s <= rec.nstep;
+      end = s == rec.nstep;
     }
+    int flags = 0;
+    bool eval = false;
     double ju = 0., ku = 0.;
     Jar jar = {0., 0., 0., 0., 0., 0., 0., 0., 0., 0., 0.};
     double e1[4] = {0., 0., 0., 0.}, e2[4] = {0., 0., 0., 0.}, Econ[4][4];
 #pragma unroll
     for (int q = 0; q < 4; q++) Econ[1][q] = Econ[2][q] = 0.;
-    /* get_jkinv at every radiating point and at the far end of the ray
-     * (src/ipolarray.c:74,143); jar_calc and the tetrad of evolve_N
-     * (src/ipolarray.c:357-384) at radiating points */
-    if ((flags & 1) || s == rec.nstep) {
-      ModelPt mp;
-      model_point_t<P>(fields, X1, X2, X3, pg, &mp);
-      int want_pol = pol && (flags & 1);
+    double K[4];
+    ModelPt mp;
+    if (live) {
+      p = step_ptr(pool, c, slot);
+      const double X1 = p[REC_X1], X2 = p[REC_X2], X3 = p[REC_X3];
+      load4(p + REC_K, K);
+      PointGeo pg;
+      point_geo<PlugT<P>::MET>(X1, X2, &pg);
+      flags = radiating_t<P>(pg) ? 1 : 0;
+      /* isolate_counterjet, src/ipolarray.c:128-136 */
+      if (C.counterjet == 1) {
+        if (X2 < (G.cstopx[2] - G.cstartx[2]) / 2) flags |= 2;
+      } else if (C.counterjet == 2) {
+        if (X2 > (G.cstopx[2] - G.cstartx[2]) / 2) flags |= 2;
+      }
+      /* get_jkinv at every radiating point and at the far end of the ray
+       * (src/ipolarray.c:74,143); jar_calc and the tetrad of evolve_N
+       * (src/ipolarray.c:357-384) at radiating points */
+      eval = (flags & 1) || end;
+      if (eval) model_point_t<P>(fields, X1, X2, X3, pg, &mp);
+    }
+    const int want_pol = pol && (flags & 1);
+    if (eval) {
       coeffs_t<P, F32>(mp, K, want_pol, EM ? EM : C.emission_type, &ju, &ku, &jar);
       if constexpr (ADJ) {
         JarGeo jg;
         jar_geo(mp, K, EM ? EM : C.emission_type, &jg);
         double *q = adj_side + ((size_t)c * IPG_CHUNK_STEPS + slot) * IPG_ADJ_DOUBLES;
-        store4(q, X1, X2, X3, jg.nu);
+        store4(q, p[REC_X1], p[REC_X2], p[REC_X3], jg.nu);
         store4(q + 4, jg.sth, jg.cth, jg.theta, (double)(jg.along | (mp.in_domain << 1)));
       }
-      if (want_pol) {
-        double Bcon[4] = {mp.Bcon[0], mp.Bcon[1], mp.Bcon[2], mp.Bcon[3]};
-        double bsq = Bcon[0] * mp.Bcov[0] + Bcon[1] * mp.Bcov[1] + Bcon[2] * mp.Bcov[2] + Bcon[3] * mp.Bcov[3];
-        if (bsq <= 0.) {
-          Bcon[0] = 0.;
-          Bcon[1] = 1.;
-          Bcon[2] = 1.;
-          Bcon[3] = 1.;
-        }
-        int tf = plasma_tetrad<PlugT<P>::MET>(mp.Ucon, K, Bcon, mp.geo.g, mp.geo, Econ, e1, e2);
-        if (isnan(mp.Ucov[0])) tf |= 8;
-        flags |= tf << 2;
-      }
     }
+    if (want_pol) {
+      double Bcon[4] = {mp.Bcon[0], mp.Bcon[1], mp.Bcon[2], mp.Bcon[3]};
+      double bsq = Bcon[0] * mp.Bcov[0] + Bcon[1] * mp.Bcov[1] + Bcon[2] * mp.Bcov[2] + Bcon[3] * mp.Bcov[3];
+      if (bsq <= 0.) {
+        Bcon[0] = 0.;
+        Bcon[1] = 1.;
+        Bcon[2] = 1.;
+        Bcon[3] = 1.;
+      }
+      int tf = plasma_tetrad<PlugT<P>::MET>(mp.Ucon, K, Bcon, mp.geo.g, mp.geo, Econ, e1, e2);
+      if (isnan(mp.Ucov[0])) tf |= 8;
+      flags |= tf << 2;
+    }
+    if (!live) continue;
     if (C.mixed) {
       /* the compact layout: coefficients in FP64, tetrad rows in FP32; dl and
        * nturns move from the geodesic state, which this pass has not yet
@@ -2008,9 +2031,9 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
    * image 1% faster, since instruction fetch is this kernel's largest stall */
 #define IPG_LAUNCH_COEF(EMT, F)                                                                                 \
   do {                                                                                                         \
-    int cb = grid_blocks(ctx, (const void *)k_coeffs<P, EMT, false, F>, threads,                              \
+    int cb = grid_blocks(ctx, (const void *)k_coeffs<P, EMT, false, F>, IPG_COEF_TPB,                              \
                          (size_t)b.n_chunks * IPG_CHUNK_STEPS);                                                \
-    k_coeffs<P, EMT, false, F><<<cb, threads, 0, b.stream>>>(b.pool, b.chunk_meta, b.cnt, b.n_chunks,         \
+    k_coeffs<P, EMT, false, F><<<cb, IPG_COEF_TPB, 0, b.stream>>>(b.pool, b.chunk_meta, b.cnt, b.n_chunks,         \
                                                              ctx->d_rays, ctx->d_fields, nullptr);             \
   } while (0)
   if constexpr (P != IPG_PLUG_ANALYTIC && IPG_COEF_EM_SPECIALIZE) {
@@ -2027,8 +2050,8 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
     }
 #undef IPG_LAUNCH_COEF
   } else {
-    int cb = grid_blocks(ctx, (const void *)k_coeffs<P>, threads, (size_t)b.n_chunks * IPG_CHUNK_STEPS);
-    k_coeffs<P><<<cb, threads, 0, b.stream>>>(b.pool, b.chunk_meta, b.cnt, b.n_chunks, ctx->d_rays, ctx->d_fields,
+    int cb = grid_blocks(ctx, (const void *)k_coeffs<P>, IPG_COEF_TPB, (size_t)b.n_chunks * IPG_CHUNK_STEPS);
+    k_coeffs<P><<<cb, IPG_COEF_TPB, 0, b.stream>>>(b.pool, b.chunk_meta, b.cnt, b.n_chunks, ctx->d_rays, ctx->d_fields,
                                               nullptr);
   }
   CK(cudaGetLastError());
@@ -2783,12 +2806,12 @@ extern "C" int ipg_trace_pixels_noalloc(const ipg_grid *g, const double *d_field
     /* the compiled kernels of a context's FP64 path, so that both give the
      * same bits for every ray */
     if (cam->emission_type == 1) {
-      int cb = na_blocks(n_sm, (const void *)k_coeffs<IPG_PLUG_IHARM, 1>, threads, (size_t)n_chunks * IPG_CHUNK_STEPS);
-      k_coeffs<IPG_PLUG_IHARM, 1><<<cb, threads, 0, stream>>>(pool, chunk_meta, cnt_d, n_chunks, rays, d_fields,
+      int cb = na_blocks(n_sm, (const void *)k_coeffs<IPG_PLUG_IHARM, 1>, IPG_COEF_TPB, (size_t)n_chunks * IPG_CHUNK_STEPS);
+      k_coeffs<IPG_PLUG_IHARM, 1><<<cb, IPG_COEF_TPB, 0, stream>>>(pool, chunk_meta, cnt_d, n_chunks, rays, d_fields,
                                                               nullptr);
     } else {
-      int cb = na_blocks(n_sm, (const void *)k_coeffs<IPG_PLUG_IHARM, 4>, threads, (size_t)n_chunks * IPG_CHUNK_STEPS);
-      k_coeffs<IPG_PLUG_IHARM, 4><<<cb, threads, 0, stream>>>(pool, chunk_meta, cnt_d, n_chunks, rays, d_fields,
+      int cb = na_blocks(n_sm, (const void *)k_coeffs<IPG_PLUG_IHARM, 4>, IPG_COEF_TPB, (size_t)n_chunks * IPG_CHUNK_STEPS);
+      k_coeffs<IPG_PLUG_IHARM, 4><<<cb, IPG_COEF_TPB, 0, stream>>>(pool, chunk_meta, cnt_d, n_chunks, rays, d_fields,
                                                               nullptr);
     }
     NA_CK(cudaGetLastError());

@@ -1380,17 +1380,20 @@ static void devgrid_derived(DevGrid *d)
   d->inv_lx2 = 1. / (d->cstopx[2] - d->cstartx[2]);
 }
 
-/* Length classes of a split wave: rays predicted at least PRED_CLASS_FACS[c]
- * times the mean length go to class c (the first class runs wide), the rest
- * to the last class. */
-#ifndef PRED_CLASS_FACS
-#define PRED_CLASS_FACS 4., 2.
-#endif
-static const double k_class_facs[] = {PRED_CLASS_FACS};
+/* Length classes of a split wave: rays predicted at least facs[c] times the
+ * mean length go to class c (the first class runs wide), the rest to the
+ * last class.  A wave of more than two resident grids of k_geodesic (512 rays
+ * per SM) is bound by the throughput of its last class, geodesics,
+ * coefficients, walk; its middle class at 2 to 4 times the mean ended later
+ * than that, so there the longest class takes rays from 2.5 times the mean
+ * and the middle one those from 1.5.  ms per image, 4 and 2 / 2.5 and 1.5:
+ * 400x400 161 / 142 (mixed tier 133 / 128), 280x280 91 / 74, 96 / 72 (128x64x64
+ * dump, mixed), 360x360 98 / 96; but 230x230 (52 900 rays) 56 / 59, 128x128 36 /
+ * 37, and unpolarized images, which end on their longest rays, 340x340 70 /
+ * 71. */
+static const double k_class_facs[] = {4., 2.}, k_class_facs_large[] = {2.5, 1.5};
 #define NB_MAX ((int)(sizeof(k_class_facs) / sizeof(k_class_facs[0])) + 1)
-#ifndef IPG_COEF_WAIT_LONGEST
-#define IPG_COEF_WAIT_LONGEST 1 /* the shorter classes' coefficient passes wait for the longest class's geodesics */
-#endif
+static_assert(sizeof(k_class_facs) == sizeof(k_class_facs_large), "the same number of classes");
 #define IPG_STARTED_MAX 1024   /* geodesic blocks of the longest class that can mark their start */
 #define IPG_STARTED_WAIT_US 2000 /* the host's wait for them */
 
@@ -1801,9 +1804,7 @@ static void wait_started(ipg_ctx *ctx, int n)
 /* One batch of a wave: a slice of a ray list, a slice of the trajectory pool
  * and its own counters, run as geodesic -> coefficients -> transfer on one
  * stream.  wide = 1 launches the two sequential kernels in 256-thread blocks,
- * whose registers fill an SM: no block of another kernel fits beside them.
- * coef_after, when set, holds the batch's coefficient pass until another
- * batch's geodesics are done. */
+ * whose registers fill an SM: no block of another kernel fits beside them. */
 struct Batch {
   const int32_t *list;
   size_t run;
@@ -1816,7 +1817,6 @@ struct Batch {
   cudaStream_t stream;
   cudaEvent_t *ev;
   int wide;
-  cudaEvent_t coef_after; /* k_coeffs waits for this event (or none) */
   int *started;           /* device view of host flags: the geodesic's blocks mark their start (or none) */
   mutable int geo_blocks; /* the geodesic's grid, as launched */
   int split;              /* a class of a split wave */
@@ -2023,8 +2023,7 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[1], b.stream));
-  if (b.coef_after) CK(cudaStreamWaitEvent(b.stream, b.coef_after, 0));
-  CK(cudaEventRecord(b.ev[4], b.stream)); /* coefficients start (after any wait) */
+  CK(cudaEventRecord(b.ev[4], b.stream)); /* coefficients start */
   /* the thermal models get a coefficient kernel compiled for the one fit
    * family the camera selects (Dexter, type 4, or Pandya, type 1): 88.6 KB
    * of code for iharm with Dexter's fits instead of 99.7 KB, and a 400x400
@@ -2093,7 +2092,7 @@ static void add_batch_stats(ipg_ctx *ctx, cudaEvent_t *ev, const unsigned long l
  * identity).  Traces every ray at PRED_EPS_SCALE times the step size without
  * storing anything and sorts the rays by that step count, longest first, into
  * ctx->d_sorted.  The sorted list is cut into up to NB_MAX length classes
- * at the thresholds k_class_facs (times the mean).  Returns the class sizes and
+ * at the thresholds facs (times the mean).  Returns the class sizes and
  * predicted step shares; *nb = 0 means: do not split (the wave is small,
  * nothing is long, or the pool looks too small to hold the wave at once). */
 #ifndef PRED_EPS_SCALE
@@ -2142,11 +2141,13 @@ static int plan_split(ipg_ctx *ctx, const int32_t *d_ij, const int32_t *list, si
    * after all are deferred to the next wave like any other */
   if (total * PRED_EPS_SCALE > (double)ctx->n_chunks * IPG_CHUNK_STEPS) return IPG_OK;
   double mean = total / (double)run;
+  const double *facs =
+      !cam->only_unpolarized && run > (size_t)ctx->n_sm * 512 ? k_class_facs_large : k_class_facs;
   int hi = LEN_BUCKETS; /* classes are bucket ranges [thr, hi) */
   size_t used = 0;
   int n = 0;
   for (int c = 0; c <= NB_MAX - 1; c++) {
-    int thr = (c < NB_MAX - 1) ? (int)(k_class_facs[c] * mean) + 1 : 0;
+    int thr = (c < NB_MAX - 1) ? (int)(facs[c] * mean) + 1 : 0;
     if (thr > hi) thr = hi;
     size_t cnt_c = 0;
     double st = 0.;
@@ -2328,17 +2329,9 @@ static int trace_core(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *d_ij, 
         bt[b].stream = ctx->bstream[b];
         bt[b].ev = ctx->bev[b];
         bt[b].wide = wide[b];
-        bt[b].coef_after = nullptr;
         bt[b].started = (b == 0 && wide[0] && nb > 1) ? ctx->d_started : nullptr;
         bt[b].geo_blocks = 0;
         bt[b].split = 1;
-        /* the shorter classes' coefficient passes wait for the longest
-         * class's geodesics: run beside them, they slow the longest rays'
-         * steps four- to eightfold (those rays' SMs hold no other block).
-         * With eight lanes per ray those end before the others' geodesics
-         * do, and waiting for them gains nothing (400x400: 154 against 156
-         * ms). */
-        if (IPG_COEF_WAIT_LONGEST && b > 0 && wide[0] && !geo_coop(ctx, ctx->plug, sizes[0])) bt[b].coef_after = ctx->bev[0][1];
         c0 += ncb;
         r0 += sizes[b];
       }

@@ -628,10 +628,8 @@ extern "C" int ipg_upload_iharm_batch(ipg_ctx *ctx, const ipg_grid *g, const dou
     M.ncell = ncell;
   }
   /* velocity and field primitives cell-major, as the single-image fields */
-  std::vector<double> aos(ncell * 6);
-  for (size_t c = 0; c < ncell; c++)
-    for (int f = 0; f < 6; f++) aos[c * 6 + f] = prims[IPG_BP_U1 + f][c];
-  CK(cudaMemcpy(M.fourv, aos.data(), ncell * 6 * sizeof(double), cudaMemcpyHostToDevice));
+  int rc = upload_fields(ctx, prims + IPG_BP_U1, 6, ncell, M.fourv);
+  if (rc) return rc;
   CK(cudaMemcpy(M.rho, prims[IPG_BP_RHO], ncell * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(M.uu, prims[IPG_BP_UU], ncell * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(M.bcode, prims[IPG_BP_BMAG], ncell * sizeof(double), cudaMemcpyHostToDevice));

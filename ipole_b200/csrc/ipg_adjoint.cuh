@@ -594,6 +594,17 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   return IPG_OK;
 }
 
+/* Maps the pages of a result array (its values stay) while the GPU works:
+ * freshly allocated, they are otherwise mapped one by one within the copy
+ * that fills it (39 MB: 8-10 ms, of which the copy itself takes 4) */
+static void touch_pages(double *p, size_t n)
+{
+  volatile double *q = p;
+  if (!p || !n) return;
+  for (size_t i = 0; i < n; i += 512) q[i] = q[i];
+  q[n - 1] = q[n - 1];
+}
+
 extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *ij, size_t n, const double *dL_dout,
                            int ckpt_interval, double *grad_ne, double *grad_thetae, double *grad_b,
                            ipg_pixel_out *out)
@@ -667,6 +678,7 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
   const int32_t *list = ctx->d_sorted;
   size_t pending = n, wave = n;
   int cur = 0;
+  bool touched = false;
   while (pending > 0) {
     size_t run = pending < wave ? pending : wave;
     size_t carry = pending - run;
@@ -684,6 +696,12 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, list == ctx->d_sorted, pool, side, n_chunks, next, first, dL, ctx->d_out, g, ncell, nextl);
     if (rc) return rc;
     CKA(cudaEventRecord(ctx->ev[1], st));
+    if (!touched) {
+      touch_pages(grad_ne, ncell);
+      touch_pages(grad_thetae, ncell);
+      touch_pages(grad_b, ncell);
+      touched = true;
+    }
     unsigned long long h[CNT_N];
     CKA(cudaMemcpyAsync(h, ctx->d_cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
     CKA(cudaStreamSynchronize(st));

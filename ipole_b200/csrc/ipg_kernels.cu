@@ -1438,6 +1438,9 @@ struct ipg_ctx {
   /* the adjoint's scratch, kept between calls (grow-only): dL/dout per
    * pixel, the cells' gradients, the walk's links */
   double *d_upload; /* upload_fields' scratch */
+  double *d_coef;   /* ipg_thermal_coefficients' workspace: coef_cap points, in use while coef_busy */
+  size_t coef_cap;
+  int coef_busy;
   double *d_adj_dl, *d_adj_g;
   int *d_adj_next, *d_adj_first;
   size_t adj_dl_cap, adj_g_cap, adj_next_cap, adj_first_cap;
@@ -1535,6 +1538,7 @@ extern "C" void ipg_destroy(ipg_ctx *ctx)
   batch_release(ctx);
   cudaFree(ctx->d_trace_extra);
   cudaFree(ctx->d_upload);
+  cudaFree(ctx->d_coef);
   cudaFree(ctx->d_adj_dl);
   cudaFree(ctx->d_adj_g);
   cudaFree(ctx->d_adj_next);
@@ -2600,6 +2604,7 @@ __global__ void k_thermal_coefficients(const double *__restrict__ in, long long 
   }
 }
 
+#define IPG_COEF_POINTS ((size_t)1 << 18) /* points per piece: 36 MB of workspace */
 extern "C" int ipg_thermal_coefficients(ipg_ctx *ctx, const double *in, size_t n, int emission_type, int precision,
                                         double *out)
 {
@@ -2608,26 +2613,46 @@ extern "C" int ipg_thermal_coefficients(ipg_ctx *ctx, const double *in, size_t n
     return IPG_E_ARG;
   if (!n) return IPG_OK;
   CK(cudaSetDevice(ctx->device));
+  /* in pieces, through a workspace that the context keeps (allocated and
+   * freed in each call it cost more than the kernel); a call that finds it
+   * in use by another thread takes one of its own */
+  const size_t piece = std::min(n, IPG_COEF_POINTS);
+  const bool own = __atomic_exchange_n(&ctx->coef_busy, 1, __ATOMIC_ACQUIRE) != 0;
   double *d = nullptr;
-  CK(cudaMalloc(&d, n * 17 * sizeof(double)));
   int rc = IPG_OK;
-  cudaError_t e = cudaMemcpyAsync(d, in, n * 5 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) {
-    const int blocks = (int)std::min<size_t>((n + 127) / 128, (size_t)ctx->n_sm * 8);
-    if (precision == IPG_FITS_FP32)
-      k_thermal_coefficients<true><<<blocks, 128, 0, ctx->stream>>>(d, (long long)n, emission_type, d + n * 5);
-    else
-      k_thermal_coefficients<false><<<blocks, 128, 0, ctx->stream>>>(d, (long long)n, emission_type, d + n * 5);
-    e = cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  if (own) {
+    e = cudaMalloc(&d, piece * 17 * sizeof(double));
+  } else {
+    if (ctx->coef_cap < piece) {
+      cudaFree(ctx->d_coef);
+      ctx->d_coef = nullptr;
+      ctx->coef_cap = 0;
+      e = cudaMalloc(&ctx->d_coef, piece * 17 * sizeof(double));
+      if (e == cudaSuccess) ctx->coef_cap = piece;
+    }
+    d = ctx->d_coef;
   }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out, d + n * 5, n * 12 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+  for (size_t at = 0; e == cudaSuccess && at < n; at += piece) {
+    const size_t m = std::min(piece, n - at);
+    e = cudaMemcpyAsync(d, in + 5 * at, m * 5 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) break;
+    const int blocks = (int)std::min<size_t>((m + 127) / 128, (size_t)ctx->n_sm * 8);
+    if (precision == IPG_FITS_FP32)
+      k_thermal_coefficients<true><<<blocks, 128, 0, ctx->stream>>>(d, (long long)m, emission_type, d + m * 5);
+    else
+      k_thermal_coefficients<false><<<blocks, 128, 0, ctx->stream>>>(d, (long long)m, emission_type, d + m * 5);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out + 12 * at, d + m * 5, m * 12 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
     snprintf(ctx->err, sizeof(ctx->err), "%s", cudaGetErrorString(e));
     rc = IPG_E_CUDA;
   }
-  cudaFree(d);
+  if (own) cudaFree(d);
+  else __atomic_store_n(&ctx->coef_busy, 0, __ATOMIC_RELEASE);
   return rc;
 }
 

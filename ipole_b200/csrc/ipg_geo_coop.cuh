@@ -393,8 +393,10 @@ __global__ void __launch_bounds__(TPB)
                     double *__restrict__ pool, int *__restrict__ chunk_prev, int2 *__restrict__ chunk_meta,
                     long long n_chunks, unsigned long long *__restrict__ counters, int queue,
                     RayRec *__restrict__ rays, int32_t *__restrict__ deferred, const int32_t *__restrict__ ray_grp,
-                    int *started = nullptr)
+                    int warps, int *started = nullptr)
 {
+  /* a wide block's other warps only hold its registers */
+  if ((int)(threadIdx.x >> 5) >= warps) return;
   if (started && threadIdx.x == 0) {
     *(volatile int *)(started + blockIdx.x) = 1;
     __threadfence_system();

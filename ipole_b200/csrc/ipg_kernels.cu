@@ -1865,7 +1865,12 @@ static bool geo_coop(const ipg_ctx *ctx, int plug, size_t n) { return plug == IP
 /* In a split wave its blocks are 384 threads wide (their registers fill an
  * SM, so that no other class's kernel runs beside them and competes for
  * instruction fetch: the 400x400 image 154 ms against 162 ms with 32-thread
- * blocks); alone, 32-thread blocks spread the warps over all schedulers. */
+ * blocks); alone, 32-thread blocks spread the warps over all schedulers.
+ * A wide block's twelve warps share four schedulers, so few rays spread over
+ * up to a quarter of the SMs, down to one working warp per scheduler: an
+ * adaptive 320x320 image 91 -> 84 ms, a sweep of 64x64 images 85 -> 81, a
+ * 128x128 image 36.9 -> 35.3 (an eighth of the SMs: 86, 86, 35.5; a half: 86,
+ * 81, 35.4). */
 #define IPG_COOP_WIDE 384
 
 template <class CS>
@@ -1877,10 +1882,17 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
 #define IPG_LAUNCH_COOP(POL, MIXED, TPB)                                                                           \
   do {                                                                                                             \
     int gb = grid_blocks(ctx, (const void *)k_geodesic_coop<POL, MIXED, TPB, CS>, TPB, n * GC_LANES);              \
+    int warps = TPB / 32;                                                                                          \
+    if (TPB == IPG_COOP_WIDE) {                                                                                    \
+      const int w = (int)((n * GC_LANES + 31) / 32), spread = std::min((w + 3) / 4, ctx->n_sm / 4);                \
+      if (gb < spread) gb = spread;                                                                                \
+      warps = std::min(warps, (w + gb - 1) / gb);                                                                  \
+    }                                                                                                              \
     if (started && gb > IPG_STARTED_MAX) gb = IPG_STARTED_MAX;                                                     \
     *blocks = gb;                                                                                                  \
     k_geodesic_coop<POL, MIXED, TPB, CS><<<gb, TPB, 0, stream>>>(d_ij, list, (int)n, pool, chunk_prev, chunk_meta, \
-                                                                 n_chunks, cnt, queue, rays, deferred, grp, started); \
+                                                                 n_chunks, cnt, queue, rays, deferred, grp, warps, \
+                                                                 started);                                         \
   } while (0)
 #define IPG_LAUNCH_COOP_T(POL, MIXED)                     \
   do {                                                    \

@@ -618,6 +618,9 @@ extern "C" int ipg_upload_iharm_batch(ipg_ctx *ctx, const ipg_grid *g, const dou
   CK(cudaSetDevice(ctx->device));
   BatchModel &M = B->m;
   const size_t ncell = (size_t)(g->n1 + 2) * (g->n2 + 2) * (g->n3 + 2);
+  int rc = upload_reserve(ctx);
+  if (rc) return rc;
+  M.have = 0; /* until every primitive is there */
   if (M.ncell != ncell) {
     batch_model_free(&M);
     CK(cudaMalloc(&M.fourv, ncell * 6 * sizeof(double)));
@@ -628,7 +631,7 @@ extern "C" int ipg_upload_iharm_batch(ipg_ctx *ctx, const ipg_grid *g, const dou
     M.ncell = ncell;
   }
   /* velocity and field primitives cell-major, as the single-image fields */
-  int rc = upload_fields(ctx, prims + IPG_BP_U1, 6, ncell, M.fourv);
+  rc = upload_fields(ctx, prims + IPG_BP_U1, 6, ncell, M.fourv);
   if (rc) return rc;
   CK(cudaMemcpy(M.rho, prims[IPG_BP_RHO], ncell * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(M.uu, prims[IPG_BP_UU], ncell * sizeof(double), cudaMemcpyHostToDevice));

@@ -1585,9 +1585,13 @@ __global__ void k_interleave(const double *__restrict__ src, long long n, int nf
  * The copies read pageable memory: they are done with the fields when they
  * return. */
 #define IPG_UPLOAD_CELLS ((size_t)1 << 20)
-static int upload_fields(ipg_ctx *ctx, const double *const *fields, int nf, size_t ncell, double *dst)
+static int upload_reserve(ipg_ctx *ctx)
 {
   if (!ctx->d_upload) CK(cudaMalloc(&ctx->d_upload, IPG_UPLOAD_CELLS * sizeof(double)));
+  return IPG_OK;
+}
+static int upload_fields(ipg_ctx *ctx, const double *const *fields, int nf, size_t ncell, double *dst)
+{
   for (size_t c0 = 0; c0 < ncell; c0 += IPG_UPLOAD_CELLS) {
     const size_t n = std::min(IPG_UPLOAD_CELLS, ncell - c0);
     for (int f = 0; f < nf; f++) {
@@ -1615,6 +1619,12 @@ extern "C" int ipg_upload_iharm(ipg_ctx *ctx, const ipg_grid *g, const double *c
   /* cell-major (AoS) layout: the 10 fields of a zone are 80 contiguous bytes
    * and the k+1 neighbour follows, so one trilinear gather reads 4 runs of
    * 160 B instead of 80 scattered words. */
+  int rc = upload_reserve(ctx);
+  if (rc) return rc;
+  /* from here until the new fields are there the context holds no dump: an
+   * upload that fails half-way must not leave the old grid over an array of
+   * another size (a known-answer model reads no fields and stays) */
+  if (ctx->plug == IPG_PLUG_IHARM) ctx->have_model = 0;
   if (ctx->d_fields && ctx->ncell != ncell) {
     cudaFree(ctx->d_fields);
     ctx->d_fields = NULL;
@@ -1623,7 +1633,7 @@ extern "C" int ipg_upload_iharm(ipg_ctx *ctx, const ipg_grid *g, const double *c
   ctx->d_trace_extra = NULL;
   if (!ctx->d_fields) CK(cudaMalloc(&ctx->d_fields, ncell * IPG_NFIELD * sizeof(double)));
   ctx->ncell = ncell;
-  int rc = upload_fields(ctx, fields, IPG_NFIELD, ncell, ctx->d_fields);
+  rc = upload_fields(ctx, fields, IPG_NFIELD, ncell, ctx->d_fields);
   if (rc) return rc;
   devgrid_from(g, &ctx->dg);
   memset(&ctx->dp, 0, sizeof(ctx->dp));

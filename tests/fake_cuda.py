@@ -1,0 +1,67 @@
+"""The library's host code on the CPU: its own objects, linked against a CUDA
+runtime without a device (fake_cudart.c).  A test is a script run in a
+process of its own, as the package loads one library per process; it finds
+``ip`` (the package), ``np``, ``C`` (ctypes), ``L`` (the loaded library with
+the runtime's fake_* controls) and the helpers below in scope.
+"""
+import os
+import subprocess
+import sys
+
+from ipole_b200 import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes as C
+import numpy as np
+import ipole_b200 as ip
+L = ip.lib()
+L.fake_log.restype = C.c_char_p
+
+def grid(n1, n2, n3):
+    g = ip.Grid()
+    g.n1, g.n2, g.n3 = n1, n2, n3
+    return g
+
+def fields(g):
+    return [np.ones((g.n1 + 2) * (g.n2 + 2) * (g.n3 + 2)) for _ in range(10)]
+
+def camera(**kw):
+    c = ip.Camera()
+    c.nx = c.ny = 64
+    c.maxnstep, c.emission_type, c.target_nturns, c.eps = 100, 4, -1, 0.01
+    for k, v in kw.items():
+        setattr(c, k, v)
+    return c
+
+def code(f, *a):
+    try:
+        f(*a)
+    except ip.IpgError as e:
+        return e.code
+    return 0
+
+def kernels():
+    return L.fake_log().decode().split()
+"""
+
+
+def library(tmp):
+    """Builds the library over the fake runtime into the folder tmp."""
+    build.build()
+    src = os.path.join(HERE, "fake_cudart.c")
+    obj, lib = os.path.join(tmp, "fake_cudart.o"), os.path.join(tmp, "libipole_fake.so")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc())))
+    objs = [os.path.join(build.BUILD, f[:f.rindex(".")] + ".o")
+            for f in ["ipg_kernels.cu", *build.CU_EXTRA, *build.HOST_SRC]]
+    subprocess.run(["gcc", "-w", "-O1", "-fPIC", "-I", os.path.join(cuda, "include"), "-c", src, "-o", obj], check=True)
+    subprocess.run(["g++", "-shared", "-fopenmp", "-o", lib, obj, *objs, "-lz", "-lm", "-Wl,-z,defs"], check=True)
+    return lib
+
+
+def run(lib, script):
+    env = dict(os.environ, IPOLE_B200_LIB=lib, PYTHONPATH=os.path.dirname(HERE))
+    r = subprocess.run([sys.executable, "-c", PRELUDE + script], env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout

@@ -1,0 +1,55 @@
+"""Failing CUDA calls in the library's host code, on the CPU over a fake CUDA
+runtime: what a call leaves behind when one of its steps fails."""
+import pytest
+
+from tests import fake_cuda
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return fake_cuda.library(str(tmp_path_factory.mktemp("fake")))
+
+
+@pytest.mark.parametrize("fn", ["cudaMalloc", "cudaMemcpyAsync"])
+@pytest.mark.parametrize("nth", [1, 2])
+def test_failed_upload_leaves_no_model(lib, fn, nth):
+    """A second upload, of a smaller dump, that fails: the next trace either
+    has the first dump whole or is refused; never the first dump's grid over
+    an array of the second's size."""
+    fake_cuda.run(lib, f"""
+for first in (grid(8, 8, 8), None):
+    with ip.Context(0, 8 << 20) as c:
+        if first is not None:
+            c.upload_arrays(first, fields(first))
+        small = grid(2, 2, 2)
+        L.fake_reset()
+        L.fake_fail(b"{fn}", {nth})
+        rc = code(c.upload_arrays, small, fields(small))
+        L.fake_reset()
+        if rc == 0:
+            continue # fewer calls than that
+        ij = np.zeros((1, 2), np.int32)
+        assert code(c.trace, camera(), ij) == ip.IPG_E_STATE, (first, rc)
+        c.upload_arrays(small, fields(small)) # and the context goes on
+        assert code(c.trace, camera(), ij) == 0
+""")
+
+
+@pytest.mark.parametrize("fn,nth", [("cudaMemcpyAsync", 3), ("cudaMemcpy", 1)])
+def test_failed_batch_upload_leaves_no_model(lib, fn, nth):
+    """the same for a batch's primitives"""
+    fake_cuda.run(lib, f"""
+g = grid(4, 4, 4)
+prims = (C.POINTER(C.c_double) * 9)(*[f.ctypes.data_as(C.POINTER(C.c_double)) for f in (fields(g) * 2)[:9]])
+up = lambda: L.ipg_upload_iharm_batch(c._h, C.byref(g), prims, C.c_double(4 / 3), C.c_double(4 / 3), C.c_double(5 / 3))
+cam, el, slot = camera(), (C.c_double * 8)(), (C.c_int * 1)(0)
+begin = lambda: L.ipg__batch_begin(c._h, C.byref(cam), 1, slot, 1, el, 1, 0)
+with ip.Context(0, 8 << 20) as c:
+    assert up() == 0 and begin() == 0
+    L.fake_reset()
+    L.fake_fail(b"{fn}", {nth})
+    assert up() != 0
+    L.fake_reset()
+    assert begin() == ip.IPG_E_STATE
+    assert up() == 0 and begin() == 0
+""")

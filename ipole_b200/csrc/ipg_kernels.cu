@@ -1450,8 +1450,11 @@ struct ipg_ctx {
 };
 static void batch_release(ipg_ctx *ctx);
 
+/* reports a failed call, and takes its error from the runtime: the check
+ * after a later call's launch must not find it again */
 static int cuda_fail(ipg_ctx *ctx, cudaError_t e, const char *where)
 {
+  cudaGetLastError();
   if (ctx) snprintf(ctx->err, sizeof(ctx->err), "%s: %s", where, cudaGetErrorString(e));
   return IPG_E_CUDA;
 }
@@ -1523,7 +1526,7 @@ extern "C" int ipg_create(ipg_ctx **out, int device, size_t pool_bytes)
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->n_sm, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) {
     free(ctx);
-    return IPG_E_CUDA;
+    return cuda_fail(NULL, e, "ipg_create");
   }
   *out = ctx;
   return IPG_OK;
@@ -2669,10 +2672,7 @@ extern "C" int ipg_thermal_coefficients(ipg_ctx *ctx, const double *in, size_t n
       e = cudaMemcpyAsync(out + 12 * at, d + m * 5, m * 12 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) {
-    snprintf(ctx->err, sizeof(ctx->err), "%s", cudaGetErrorString(e));
-    rc = IPG_E_CUDA;
-  }
+  if (e != cudaSuccess) rc = cuda_fail(ctx, e, "ipg_thermal_coefficients");
   if (own) cudaFree(d);
   else __atomic_store_n(&ctx->coef_busy, 0, __ATOMIC_RELEASE);
   return rc;

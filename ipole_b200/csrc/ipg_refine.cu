@@ -367,6 +367,7 @@ __global__ void __launch_bounds__(SCAN_TPB) k_scatter(const int32_t *flags, int 
   do {                                                                                       \
     cudaError_t e_ = (call);                                                                 \
     if (e_ != cudaSuccess) {                                                                 \
+      cudaGetLastError(); /* reported here, not by the next call's check */                  \
       char m_[400];                                                                          \
       snprintf(m_, sizeof(m_), "%s: %s", #call, cudaGetErrorString(e_));                     \
       ipg__set_error(ctx, m_);                                                               \

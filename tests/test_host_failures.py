@@ -53,3 +53,22 @@ with ip.Context(0, 8 << 20) as c:
     assert begin() == ip.IPG_E_STATE
     assert up() == 0 and begin() == 0
 """)
+
+
+@pytest.mark.parametrize("call", ["c.upload_arrays(big, fields(big))", "c.trace(camera(), np.zeros((9, 2), np.int32))",
+                                  "c.thermal_coefficients(np.ones((7, 5)))"])
+def test_recovers_after_out_of_memory(lib, call):
+    """a call that finds no memory fails by itself: the next upload, trace and
+    fits, which have what they need, are not refused for it"""
+    fake_cuda.run(lib, f"""
+with ip.Context(0, 8 << 20) as c:
+    g, big = grid(2, 2, 2), grid(3, 3, 3)
+    c.upload_arrays(g, fields(g))
+    def failing():
+        {call}
+    L.fake_fail(b"cudaMalloc", 1)
+    assert code(failing) == ip.IPG_E_CUDA
+    assert code(c.upload_arrays, g, fields(g)) == 0
+    assert code(c.trace, camera(), np.zeros((9, 2), np.int32)) == 0
+    assert code(c.thermal_coefficients, np.ones((7, 5))) == 0
+""")

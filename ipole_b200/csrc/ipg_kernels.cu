@@ -2640,9 +2640,13 @@ extern "C" int ipg_thermal_coefficients(ipg_ctx *ctx, const double *in, size_t n
   CK(cudaSetDevice(ctx->device));
   /* in pieces, through a workspace that the context keeps (allocated and
    * freed in each call it cost more than the kernel); a call that finds it
-   * in use by another thread takes one of its own */
-  const size_t piece = std::min(n, IPG_COEF_POINTS);
-  const bool own = __atomic_exchange_n(&ctx->coef_busy, 1, __ATOMIC_ACQUIRE) != 0;
+   * in use by another thread takes one of its own.  Where the result lies
+   * over the points, a piece's result would overwrite later pieces' points:
+   * such a call goes as one piece */
+  const bool whole = n > IPG_COEF_POINTS && (uintptr_t)in < (uintptr_t)(out + 12 * n) &&
+                     (uintptr_t)out < (uintptr_t)(in + 5 * n);
+  const size_t piece = whole ? n : std::min(n, IPG_COEF_POINTS);
+  const bool own = whole || __atomic_exchange_n(&ctx->coef_busy, 1, __ATOMIC_ACQUIRE) != 0;
   double *d = nullptr;
   int rc = IPG_OK;
   cudaError_t e = cudaSuccess;

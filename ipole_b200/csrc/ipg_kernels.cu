@@ -1585,8 +1585,7 @@ __global__ void k_interleave(const double *__restrict__ src, long long n, int nf
  * in pieces of IPG_UPLOAD_CELLS through a scratch that the context keeps (8
  * MiB), and the device interleaves.  Interleaved by a host core, the 560 000
  * cells of a 128x64x64 dump took 20 ms before the copy (4 ms) could start.
- * The copies read pageable memory: they are done with the fields when they
- * return. */
+ * Returns when the copies are done with the fields. */
 #define IPG_UPLOAD_CELLS ((size_t)1 << 20)
 static int upload_reserve(ipg_ctx *ctx)
 {
@@ -1595,16 +1594,20 @@ static int upload_reserve(ipg_ctx *ctx)
 }
 static int upload_fields(ipg_ctx *ctx, const double *const *fields, int nf, size_t ncell, double *dst)
 {
-  for (size_t c0 = 0; c0 < ncell; c0 += IPG_UPLOAD_CELLS) {
+  cudaError_t e = cudaSuccess;
+  for (size_t c0 = 0; e == cudaSuccess && c0 < ncell; c0 += IPG_UPLOAD_CELLS) {
     const size_t n = std::min(IPG_UPLOAD_CELLS, ncell - c0);
-    for (int f = 0; f < nf; f++) {
-      CK(cudaMemcpyAsync(ctx->d_upload, fields[f] + c0, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    for (int f = 0; e == cudaSuccess && f < nf; f++) {
+      e = cudaMemcpyAsync(ctx->d_upload, fields[f] + c0, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+      if (e != cudaSuccess) break;
       k_interleave<<<4 * ctx->n_sm, 256, 0, ctx->stream>>>(ctx->d_upload, (long long)n, nf, f, dst + c0 * nf);
-      CK(cudaGetLastError());
+      e = cudaGetLastError();
     }
   }
-  CK(cudaStreamSynchronize(ctx->stream));
-  return IPG_OK;
+  /* (after a failure too: copies from page-locked fields may be in flight) */
+  const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? IPG_OK : cuda_fail(ctx, e, "upload of the fields");
 }
 
 extern "C" int ipg_upload_iharm(ipg_ctx *ctx, const ipg_grid *g, const double *const fields[IPG_NFIELD])
@@ -2675,7 +2678,10 @@ extern "C" int ipg_thermal_coefficients(ipg_ctx *ctx, const double *in, size_t n
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(out + 12 * at, d + m * 5, m * 12 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  /* (after a failure too: the copies in flight use the caller's arrays and
+   * the workspace) */
+  const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) rc = cuda_fail(ctx, e, "ipg_thermal_coefficients");
   if (own) cudaFree(d);
   else __atomic_store_n(&ctx->coef_busy, 0, __ATOMIC_RELEASE);

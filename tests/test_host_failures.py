@@ -72,3 +72,22 @@ with ip.Context(0, 8 << 20) as c:
     assert code(c.trace, camera(), np.zeros((9, 2), np.int32)) == 0
     assert code(c.thermal_coefficients, np.ones((7, 5))) == 0
 """)
+
+
+@pytest.mark.parametrize("call", ["c.upload_arrays(g, fields(g))",
+                                  "c.thermal_coefficients(np.ones(((1 << 18) + 9, 5)))"])
+@pytest.mark.parametrize("fn", ["cudaGetLastError", "cudaMemcpyAsync"])
+def test_failed_call_waits_for_its_copies(lib, call, fn):
+    """a call that fails between its copies returns after the ones in flight,
+    which use the caller's arrays, are done"""
+    fake_cuda.run(lib, f"""
+with ip.Context(0, 8 << 20) as c:
+    g = grid(2, 2, 2)
+    def failing():
+        {call}
+    failing()
+    L.fake_reset()
+    L.fake_fail(b"{fn}", 2)
+    assert code(failing) == ip.IPG_E_CUDA
+    assert L.fake_inflight() == 0
+""")

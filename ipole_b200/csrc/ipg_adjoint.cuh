@@ -693,8 +693,12 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     }
     CKA(cudaEventRecord(ctx->ev[0], st));
     const int em = cam->emission_type;
-    rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, list == ctx->d_sorted, pool, side, n_chunks, next, first, dL, ctx->d_out, g, ncell, nextl);
-    if (rc) return rc;
+    rc = adjoint_wave(ctx, em, ctx->d_ij, list, run, list == ctx->d_sorted, pool, side, n_chunks, next, first, dL,
+                      ctx->d_out, g, ncell, nextl);
+    if (rc) {
+      wave_stop(ctx);
+      return rc;
+    }
     CKA(cudaEventRecord(ctx->ev[1], st));
     if (!touched) {
       touch_pages(grad_ne, ncell);

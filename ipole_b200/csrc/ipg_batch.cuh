@@ -1045,6 +1045,7 @@ extern "C" int ipg__batch_trace(ipg_ctx *ctx, const ipg_batch_items *it, unsigne
   if (rc) return rc;
   BatchRider R = {0, 0, false, false};
   rc = batch_waves(ctx, it, steps_left, R);
+  if (rc) wave_stop(ctx);
   if (R.launched) {
     /* the context's stream continues after the waves; on an early return
      * the class's geodesics, which write into the pool, end before it */

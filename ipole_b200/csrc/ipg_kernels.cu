@@ -2045,6 +2045,11 @@ static int walk_join(ipg_ctx *ctx, cudaStream_t st)
   return IPG_OK;
 }
 
+/* After a wave that failed: its second stream (of the geodesics' head, or of
+ * the walk behind one), which the context's stream may not wait for, ends
+ * before the call returns */
+static void wave_stop(ipg_ctx *ctx) { cudaStreamSynchronize(ctx->bstream[NB_MAX - 1]); }
+
 template <bool S32, int RM>
 static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
 {

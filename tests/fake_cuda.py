@@ -18,6 +18,7 @@ import numpy as np
 import ipole_b200 as ip
 L = ip.lib()
 L.fake_log.restype = C.c_char_p
+L.fake_inflight.argtypes = [C.c_void_p]
 
 def grid(n1, n2, n3):
     g = ip.Grid()

@@ -328,8 +328,9 @@ int ipg_trace_ray(ipg_ctx *ctx, const ipg_camera *cam, int i, int j, size_t max_
 int ipg_upload_trace_fields(ipg_ctx *ctx, const double *const extra[3]);
 
 /* Kernel statistics of the last trace call: total ray-steps of the geodesic
- * pass, steps inside the radiating region, number of kernel launches and
- * pool waves, the device time (ms, CUDA events) of the geodesic, coefficient
+ * pass, steps inside the radiating region, number of launches of the ray
+ * kernels (length prediction and its sort, geodesics, coefficients, walks,
+ * the adjoint's passes) and pool waves, the device time (ms, CUDA events) of the geodesic, coefficient
  * and transfer kernels, summed over the batches of a wave (batches run
  * concurrently, so these can add up to more than the call), the time of the
  * ray-length prediction, and the device time of the whole call. */

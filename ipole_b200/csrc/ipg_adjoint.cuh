@@ -531,6 +531,7 @@ static int launch_adj_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, double
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
   k_adj_walk<G><<<wb, 32, sm, st>>>(list, (int)n, pool, next, first, ctx->d_rays, dL, cnt, queue);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -564,6 +565,7 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
     k_coeffs<IPG_PLUG_IHARM, 4, true><<<cb, IPG_COEF_TPB, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays,
                                                               ctx->d_fields, side);
   }
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev[3], st));
   /* the longest rays' walks with 32 lanes beside the others' (walk_head) */
@@ -579,6 +581,7 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   if (rc || (head && (rc = walk_join(ctx, st)))) return rc;
   CK(cudaEventRecord(ctx->ev[4], st));
   k_adj_link<<<4 * ctx->n_sm, 256, 0, st>>>(ctx->d_chunk_prev, ctx->d_chunk_meta, cnt, n_chunks, next, first);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   if (head) {
     if ((rc = walk_fork(ctx, st, &sr))) return rc;
@@ -590,6 +593,7 @@ static int adjoint_wave(ipg_ctx *ctx, int em, const int32_t *d_ij, const int32_t
   int sb = grid_blocks(ctx, (const void *)k_adj_scatter, IPG_SCAT_TPB, (size_t)n_chunks * IPG_CHUNK_STEPS);
   k_adj_scatter<<<sb, IPG_SCAT_TPB, 0, st>>>(pool, ctx->d_chunk_meta, cnt, n_chunks, ctx->d_rays, side, ctx->d_fields, g,
                                         g + ncell, g + 2 * ncell);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -725,7 +729,6 @@ extern "C" int ipg_adjoint(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *i
     ctx->stats.adj_scatter_ms += t[4];
     ctx->stats.ray_steps += h[CNT_STEPS];
     ctx->stats.radiating_steps += h[CNT_RAD];
-    ctx->stats.launches += 5;
     ctx->stats.waves += 1;
     size_t deferred = (size_t)h[CNT_DEFER];
     if (deferred == pending) {

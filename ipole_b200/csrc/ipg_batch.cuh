@@ -774,6 +774,7 @@ static int batch_ws_reserve(ipg_ctx *ctx, BatchWs &w, size_t n_geo, size_t n_xf)
     int tb = grid_blocks(ctx, (const void *)k_xfer_batch<TPB, S32, RMC>, TPB, nt);                                 \
     k_xfer_batch<TPB, S32, RMC><<<tb, TPB, 0, sx>>>(tail, (int)nt, pool, side, G, ctx->d_chunk_prev, W.rays,       \
                                                     it->xf_geo, it->xf_slot, it->geo_grp, it->xf_out, W.cnt, xnext); \
+    ctx->stats.launches++;                                                                                         \
   } while (0)
 
 /* Trace one level of a batch: every geodesic item once, then its step
@@ -853,6 +854,7 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
       k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CamTable><<<lb, 256, 0, sr>>>(
           it->geo_ij, it->geo_order, nl, pool, ctx->d_chunk_prev, ctx->d_chunk_meta, R.cl, W.cnt_long, W.rays_long,
           W.gdef_long, it->geo_grp, ctx->d_started);
+      ctx->stats.launches++;
       CK(cudaGetLastError());
     }
     /* the waves' blocks are launched once the class's SM-filling blocks are
@@ -949,6 +951,7 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
       }
     }
 #undef IPG_LAUNCH_BCOEF
+    ctx->stats.launches++;
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[2], st));
     /* (items of the longest rays come first: xf_order follows the sorted
@@ -1001,7 +1004,6 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
     B->call_items += (double)pend_x;
     ctx->stats.ray_steps += h[CNT_STEPS];
     ctx->stats.radiating_steps += h[CNT_RAD];
-    ctx->stats.launches += 3;
     ctx->stats.waves += 1;
     if (steps_left) {
       const unsigned long long used = h[CNT_STEPS] + h[CNT_XSTEPS];

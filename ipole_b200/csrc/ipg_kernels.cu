@@ -1924,6 +1924,7 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
   }
 #undef IPG_LAUNCH_COOP_T
 #undef IPG_LAUNCH_COOP
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -1966,6 +1967,7 @@ static int launch_geo_wave(ipg_ctx *ctx, int unpol, int mixed, const int32_t *d_
   k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CS><<<gb, 128, 0, st>>>(
       d_ij, list ? list + head : list, (int)(n - head), pool, chunk_prev, chunk_meta, n_chunks, cnt, rays, deferred,
       grp);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   if (head) CK(cudaStreamWaitEvent(st, ctx->ev_join[NB_MAX - 1], 0));
   return IPG_OK;
@@ -1987,6 +1989,7 @@ static int launch_walk_g(ipg_ctx *ctx, const int32_t *list, size_t n, const doub
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int wb = grid_blocks(ctx, fn, 32, n * G, sm);
   k_walk<G, S32, RM, ADJ, BATCH><<<wb, 32, sm, stream>>>(list, (int)n, pool, chunk_prev, rays, d_out, cnt, queue, wa);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -2058,6 +2061,7 @@ static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
     int tb = grid_blocks(ctx, (const void *)k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM>, xthreads, b.run);
     k_transfer<IPG_XFER_WIDE, IPG_XFER_MINB, S32, RM><<<tb, xthreads, 0, b.stream>>>(
         b.list, (int)b.run, b.pool, b.chunk_prev, ctx->d_rays, d_out, b.cnt);
+    ctx->stats.launches++;
     CK(cudaGetLastError());
     return IPG_OK;
   }
@@ -2086,6 +2090,7 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
     k_geodesic<P, 256, IPG_GEO_MINB><<<gb, gthreads, 0, b.stream>>>(d_ij, b.list, (int)b.run, b.pool, b.chunk_prev,
                                                                     b.chunk_meta, b.n_chunks, b.cnt, ctx->d_rays,
                                                                     b.deferred, nullptr, b.started);
+    ctx->stats.launches++;
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[1], b.stream));
@@ -2119,6 +2124,7 @@ static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg
     k_coeffs<P><<<cb, IPG_COEF_TPB, 0, b.stream>>>(b.pool, b.chunk_meta, b.cnt, b.n_chunks, ctx->d_rays, ctx->d_fields,
                                               nullptr);
   }
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   CK(cudaEventRecord(b.ev[2], b.stream));
   int rc = ctx->step32 ? (ctx->rec_mixed ? launch_transfer<true, 1>(ctx, b, d_out) : launch_transfer<true, 0>(ctx, b, d_out))
@@ -2151,7 +2157,6 @@ static void add_batch_stats(ipg_ctx *ctx, cudaEvent_t *ev, const unsigned long l
   ctx->stats.transfer_ms += c;
   ctx->stats.ray_steps += cnt[CNT_STEPS];
   ctx->stats.radiating_steps += cnt[CNT_RAD];
-  ctx->stats.launches += 3;
 }
 
 /* Length prediction and split of a wave (rays run..: the list, or the
@@ -2172,6 +2177,7 @@ static void launch_count_t(ipg_ctx *ctx, int threads, const int32_t *d_ij, const
   int gb = grid_blocks(ctx, (const void *)k_geodesic_count<P>, threads, run);
   k_geodesic_count<P><<<gb, threads, 0, ctx->stream>>>(d_ij, list, (int)run, PRED_EPS_SCALE, cap, ctx->d_pred,
                                                        counter, nullptr);
+  ctx->stats.launches++;
 }
 #define SPLIT_MIN_RAYS 4096
 
@@ -2195,6 +2201,7 @@ static int plan_split(ipg_ctx *ctx, const int32_t *d_ij, const int32_t *list, si
   int sb = (int)((run + 255) / 256);
   if (sb > 4 * ctx->n_sm) sb = 4 * ctx->n_sm;
   k_len_hist<<<sb, 256, 0, ctx->stream>>>(ctx->d_pred, (int)run, 0, ctx->d_len_hist);
+  ctx->stats.launches++;
   CK(cudaGetLastError());
   std::vector<int> hist(LEN_BUCKETS);
   CK(cudaMemcpyAsync(hist.data(), ctx->d_len_hist, LEN_BUCKETS * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2233,6 +2240,7 @@ static int plan_split(ipg_ctx *ctx, const int32_t *d_ij, const int32_t *list, si
   if (n < 2 || sizes[n - 1] == run) return IPG_OK;
   k_len_scan<<<1, LEN_SCAN_THREADS, 0, ctx->stream>>>(ctx->d_len_hist);
   k_len_scatter<<<sb, 256, 0, ctx->stream>>>(list, ctx->d_pred, (int)run, 0, ctx->d_len_hist, ctx->d_sorted);
+  ctx->stats.launches += 2;
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev_pred[1], ctx->stream));
   *nb = n;
@@ -2261,6 +2269,7 @@ static int sort_by_length(ipg_ctx *ctx, const int32_t *d_ij, size_t n, const ipg
   k_len_hist<<<sb, 256, 0, ctx->stream>>>(ctx->d_pred, (int)n, 0, ctx->d_len_hist);
   k_len_scan<<<1, LEN_SCAN_THREADS, 0, ctx->stream>>>(ctx->d_len_hist);
   k_len_scatter<<<sb, 256, 0, ctx->stream>>>(NULL, ctx->d_pred, (int)n, 0, ctx->d_len_hist, ctx->d_sorted);
+  ctx->stats.launches += 3;
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -2311,6 +2320,7 @@ extern "C" int ipg__batch_sort_geo(ipg_ctx *ctx, const int32_t *geo_ij, const in
   }
   k_len_scan<<<1, LEN_SCAN_THREADS, 0, ctx->stream>>>(ctx->d_len_hist);
   k_len_scatter<<<sb, 256, 0, ctx->stream>>>(NULL, pred, (int)n, 0, ctx->d_len_hist, sorted);
+  ctx->stats.launches += 4; /* with the prediction */
   CK(cudaGetLastError());
   return IPG_OK;
 }
@@ -2367,7 +2377,6 @@ static int trace_core(ipg_ctx *ctx, const ipg_camera *cam, const int32_t *d_ij, 
       if (!nb) split_ok = 0; /* later waves are this wave's leftovers */
     }
     if (nb) {
-      ctx->stats.launches += 4;
       /* pool shares: the predicted share of steps with a margin for the
        * longer classes (their rays are the hardest to predict); the last
        * class gets the rest */

@@ -47,6 +47,35 @@ def kernels():
     return L.fake_log().decode().split()
 """
 
+# an adjoint of more rays than one launch gives eight lanes each
+ADJOINT = """
+g = grid(2, 2, 2)
+ij = np.zeros((6000, 2), np.int32)
+c.upload_arrays(g, fields(g))
+def call():
+    return code(c.adjoint, camera(), ij, np.zeros((len(ij), 4)), 64)
+"""
+# a level of a batch: one camera, n geodesics with two instances each
+BATCH = """
+g = grid(2, 2, 2)
+prims = (C.POINTER(C.c_double) * 9)(*[f.ctypes.data_as(C.POINTER(C.c_double)) for f in (fields(g) * 2)[:9]])
+cam, el, slot = camera(), (C.c_double * 8)(), (C.c_int * 2)(0, 0)
+class Items(C.Structure):
+    _fields_ = [("n_geo", C.c_size_t), ("geo_ij", C.c_void_p), ("geo_grp", C.c_void_p), ("geo_mask", C.c_void_p),
+                ("n_xf", C.c_size_t), ("xf_geo", C.c_void_p), ("xf_slot", C.c_void_p), ("xf_out", C.c_void_p),
+                ("xf_order", C.c_void_p), ("geo_order", C.c_void_p), ("n_long", C.c_size_t),
+                ("long_steps", C.c_double), ("pred_steps", C.c_double)]
+buf = np.zeros(1 << 20, np.int32)
+def call(n=6000):
+    it = Items(n, *[buf.ctypes.data] * 3, 2 * n, *[buf.ctypes.data] * 5, 0, 0., 0.)
+    return L.ipg__batch_trace(c._h, C.byref(it), None)
+def begin():
+    assert L.ipg_upload_iharm_batch(c._h, C.byref(g), prims, C.c_double(4 / 3), C.c_double(4 / 3),
+                                    C.c_double(5 / 3)) == 0
+    assert L.ipg__batch_begin(c._h, C.byref(cam), 1, slot, 2, el, 1, 0) == 0
+begin()
+"""
+
 
 def library(tmp):
     """Builds the library over the fake runtime into the folder tmp."""

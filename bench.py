@@ -498,8 +498,7 @@ def bench_batched(ip, ctx, model, dump, args, world, stream, single_ms):
         ctx.set_step_precision(ip.IPG_STEP_FP32 if step32 else ip.IPG_STEP_FP64)
         ctx.set_fit_precision(ip.IPG_FITS_FP32 if fits32 else ip.IPG_FITS_FP64)
         ctx.set_record_precision(ip.IPG_RECORDS_MIXED if fits32 else ip.IPG_RECORDS_FP64)
-        # untimed: the first two calls of a batch shape try both transfer
-        # block sizes (the context's tuner), the timed ones use the faster
+        # untimed: first launches and allocations
         for _ in range(2):
             ctx.render_batch(ps, model)
         torch.cuda.synchronize()
@@ -539,8 +538,7 @@ def bench_batched(ip, ctx, model, dump, args, world, stream, single_ms):
             for ii, inc in enumerate(BATCH_INCL):
                 ps96 += batch_params(ip, dump, args.m_unit, BATCH_RES[(fi + ii) % 3], inc, fq, refine=True)
         # FP64, then the mixed tier (FP32 step, FP32 fit shapes, compact
-        # records); each timed on its second call (the first tunes the
-        # transfer's block size for the batch's shape)
+        # records); each timed on its second call (the first allocates)
         for tag, mixed in (("workload_96", False), ("workload_96_mixed", True)):
             ctx.set_step_precision(ip.IPG_STEP_FP32 if mixed else ip.IPG_STEP_FP64)
             ctx.set_fit_precision(ip.IPG_FITS_FP32 if mixed else ip.IPG_FITS_FP64)

@@ -430,8 +430,13 @@ __device__ __forceinline__ bool xb_fetch(XbLane &L, const int32_t *__restrict__ 
   }
 }
 
-template <int TPB, bool S32, bool RM = false>
-__global__ void __launch_bounds__(TPB, 1)
+/* Blocks of 128: with 256 the walk of a batch (transfer_ms, ms) is no
+ * faster beyond the noise and up to a fifth slower, 128 / 256: 8 instances of 160x160 25.3 / 29.3
+ * (mixed tier 28.6 / 28.3), of 400x400 139.4 / 139.0, two of 240x240 29.2 /
+ * 32.5 (28.8 / 30.6), 24 of 128x128 in the mixed tier 45.0 / 45.2 */
+#define IPG_XB_TPB 128
+template <bool S32, bool RM = false>
+__global__ void __launch_bounds__(IPG_XB_TPB, 1)
     k_xfer_batch(const int32_t *__restrict__ list, int n_list, const double *__restrict__ pool,
                  const double *__restrict__ side, int G, const int *__restrict__ chunk_prev,
                  const RayRec *__restrict__ rays, const int32_t *__restrict__ xf_geo,
@@ -553,13 +558,6 @@ struct BatchState {
   BatchWs w;
   int G; /* instance slots per group of the current batch */
   int emission_type, step32, unpol, rec_mixed;
-  int xfer_threads; /* transfer block size (128 or 256) */
-  /* the transfer block size is tuned per batch shape (slots per group,
-   * groups): the first call of a shape runs 128 threads, the second 256,
-   * and later calls keep the one whose transfer took less time per
-   * transfer item (the images do not depend on it: one lane per item) */
-  int tune_G, tune_ngrp, tune_calls;
-  double tune_ms[2], tune_items[2], call_xfer_ms, call_items;
 };
 
 static void batch_ws_free(BatchWs *w)
@@ -708,25 +706,6 @@ extern "C" int ipg__batch_begin(ipg_ctx *ctx, const ipg_camera *grp_cam, int ngr
   B->unpol = unpol;
   B->step32 = step32;
   B->rec_mixed = ctx->rec_mixed;
-  /* block-size tuning: close the previous call's sample, pick this call's */
-  if (B->tune_calls > 0 && B->tune_calls <= 2 && B->call_items > 0) {
-    B->tune_ms[B->tune_calls - 1] = B->call_xfer_ms;
-    B->tune_items[B->tune_calls - 1] = B->call_items;
-  }
-  if (G != B->tune_G || ngrp != B->tune_ngrp) {
-    B->tune_G = G;
-    B->tune_ngrp = ngrp;
-    B->tune_calls = 0;
-  }
-  if (B->tune_calls < 2) {
-    B->xfer_threads = B->tune_calls == 0 ? 128 : 256;
-  } else if (B->tune_calls == 2) {
-    const double r128 = B->tune_ms[0] / fmax(B->tune_items[0], 1.), r256 = B->tune_ms[1] / fmax(B->tune_items[1], 1.);
-    B->xfer_threads = r256 < r128 ? 256 : 128;
-  }
-  if (B->tune_calls <= 2) B->tune_calls++;
-  B->call_xfer_ms = 0.;
-  B->call_items = 0.;
   memset(&ctx->stats, 0, sizeof(ctx->stats));
   return IPG_OK;
 }
@@ -769,11 +748,12 @@ static int batch_ws_reserve(ipg_ctx *ctx, BatchWs &w, size_t n_geo, size_t n_xf)
  * wave: 6 400 items 6.4 / 7.7, 32 768 items 13.9 / 15.7 (mixed tier 20.5 /
  * 21.7), 80 000 items 21.4 / 16.8 (27.3 / 20.9), 204 800 items 51 / 25.5. */
 #define IPG_XB_LANE 300
-#define IPG_LAUNCH_XB(TPB, S32, RMC)                                                                                \
+#define IPG_LAUNCH_XB(S32, RMC)                                                                                     \
   do {                                                                                                             \
-    int tb = grid_blocks(ctx, (const void *)k_xfer_batch<TPB, S32, RMC>, TPB, nt);                                 \
-    k_xfer_batch<TPB, S32, RMC><<<tb, TPB, 0, sx>>>(tail, (int)nt, pool, side, G, ctx->d_chunk_prev, W.rays,       \
-                                                    it->xf_geo, it->xf_slot, it->geo_grp, it->xf_out, W.cnt, xnext); \
+    int tb = grid_blocks(ctx, (const void *)k_xfer_batch<S32, RMC>, IPG_XB_TPB, nt);                               \
+    k_xfer_batch<S32, RMC><<<tb, IPG_XB_TPB, 0, sx>>>(tail, (int)nt, pool, side, G, ctx->d_chunk_prev, W.rays,     \
+                                                      it->xf_geo, it->xf_slot, it->geo_grp, it->xf_out, W.cnt,     \
+                                                      xnext);                                                      \
     ctx->stats.launches++;                                                                                         \
   } while (0)
 
@@ -813,7 +793,6 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
   if (n_chunks < 16) return IPG_E_NOMEM;
   double *pool = ctx->d_pool;
   double *side = ctx->d_pool + (size_t)n_chunks * IPG_CHUNK_STEPS * IPG_STEP_DOUBLES;
-  const int threads = 128;
   const void *geo_fn = (const void *)k_geodesic<IPG_PLUG_IHARM, 256, IPG_GEO_MINB, false, CamTable>;
   cudaStream_t st = ctx->stream; /* the waves */
   size_t pend_g = it->n_geo, pend_x = it->n_xf;
@@ -971,10 +950,8 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
       if ((rc = launch_walk<S32, RMC, false, true>(ctx, tail, nt, pool, ctx->d_chunk_prev, W.rays, it->xf_out,       \
                                                    W.cnt, sx, CNT_NEXT_T, wa)))                                      \
         return rc;                                                                                                   \
-    } else if (B->xfer_threads == 256) {                                                                             \
-      IPG_LAUNCH_XB(256, S32, RMC);                                                                                  \
     } else {                                                                                                         \
-      IPG_LAUNCH_XB(128, S32, RMC);                                                                                  \
+      IPG_LAUNCH_XB(S32, RMC);                                                                                       \
     }                                                                                                                \
   } while (0)
     if (B->rec_mixed) {
@@ -1000,8 +977,6 @@ static int batch_waves(ipg_ctx *ctx, const ipg_batch_items *it, unsigned long lo
     ctx->stats.coeffs_ms += b;
     ctx->stats.transfer_ms += c;
     ctx->stats.wall_ms += a + b + c;
-    B->call_xfer_ms += c;
-    B->call_items += (double)pend_x;
     ctx->stats.ray_steps += h[CNT_STEPS];
     ctx->stats.radiating_steps += h[CNT_RAD];
     ctx->stats.waves += 1;

@@ -146,37 +146,7 @@ __constant__ DevCam c_cam;
 #define IPG_BATCH_MAX_GROUPS 64
 __constant__ DevCam c_cams[IPG_BATCH_MAX_GROUPS];
 
-/* --------------------------------------------------------------------- */
-/* small helpers                                                           */
-/* --------------------------------------------------------------------- */
-/* q^n for 0 <= n < 128 by binary powering, without branches */
-__device__ __forceinline__ double ipow_int(double q, int n)
-{
-  double r = 1.0, b = q;
-#pragma unroll
-  for (int k = 0; k < 7; k++) {
-    r *= (n & 1) ? b : 1.0;
-    b *= b;
-    n >>= 1;
-  }
-  return r;
-}
-
-/* q^(alpha-1) of the FMKS polar map */
-__device__ __forceinline__ double fmks_pow_am1(double q)
-{
-  const DevGrid &G = c_grid;
-  return (G.alpha_int >= 0) ? ipow_int(q, G.alpha_int) : pow(q, G.poly_alpha - 1.);
-}
-
-/* exp(d) and sin/cos(d) for |d| < 1e-5 (Taylor; exact to rounding) */
-__device__ __forceinline__ double expm_small(double d) { return d * (1. + d * (0.5 + d * (1. / 6.))); }
-__device__ __forceinline__ void sincos_small(double d, double *s, double *c)
-{
-  double d2 = d * d;
-  *s = d * (1. - d2 * (1. / 6.));
-  *c = 1. - 0.5 * d2;
-}
+#include "ipg_connection.cuh"
 
 /* --------------------------------------------------------------------- */
 /* FMKS metric (src/coordinates.c:46-97, 175-239, 263-305)                 */
@@ -184,22 +154,6 @@ __device__ __forceinline__ void sincos_small(double d, double *s, double *c)
 struct Met {  /* symmetric; g02 = g23 = 0 in FMKS */
   double g00, g01, g03, g11, g12, g13, g22, g33;
 };
-
-/* X2-dependent parts of theta(X1,X2) and its Jacobian */
-struct X2P {
-  double S2, C2, y, P, P1;  /* sin 2piX2, cos 2piX2, 2X2-1, q^alpha, q^(alpha-1), q = y/xt */
-};
-
-__device__ __forceinline__ void x2_parts_from(double X2, double S2, double C2, X2P *o)
-{
-  const DevGrid &G = c_grid;
-  o->S2 = S2;
-  o->C2 = C2;
-  o->y = 2. * X2 - 1.;
-  double q = o->y * G.inv_xt;
-  o->P1 = fmks_pow_am1(q);
-  o->P = o->P1 * q;
-}
 
 /* theta, dtheta/dX1 (J21) and dtheta/dX2 (J22) from the parts;
  * E = exp(mks_smooth (startx1 - X1)) */
@@ -238,38 +192,8 @@ __device__ __forceinline__ Met met_from(double r, double sth, double cth, double
   return m;
 }
 
-/* met_from at a point a finite-difference offset away from a centre where
- * rho^2 = rho2c and 1/rho^2 = irho2c are known: 1/rho^2 from the centre's by
- * 1/(1+e) = 1 - e(1 - e), e ~ 1e-7 (the e^3 term is below rounding), which
- * saves the division of each offset metric. */
-__device__ __forceinline__ Met met_from_near(double r, double sth, double cth, double J21, double J22, double rho2c,
-                                             double irho2c)
-{
-  const double a = c_grid.a;
-  double s2 = sth * sth;
-  double rho2 = r * r + a * a * cth * cth;
-  double e = (rho2 - rho2c) * irho2c;
-  double t = 2. * r * (irho2c * (1. - e * (1. - e)));
-  double G00 = -1. + t, G01 = t, G03 = -a * s2 * t, G11 = 1. + t, G13 = -a * s2 * (1. + t);
-  double G22 = rho2, G33 = s2 * (rho2 + a * a * s2 * (1. + t));
-  Met m;
-  m.g00 = G00;
-  m.g01 = G01 * r;
-  m.g03 = G03;
-  m.g11 = G11 * r * r + G22 * J21 * J21;
-  m.g12 = G22 * J21 * J22;
-  m.g13 = G13 * r;
-  m.g22 = G22 * J22 * J22;
-  m.g33 = G33;
-  return m;
-}
-
 /* Closed-form g^{mu nu} of FMKS Kerr-Schild (the reference inverts gcov by LU,
  * src/geometry.c:54-64, 252-287; both agree to rounding). */
-struct Gcon {
-  double u00, u01, u02, u11, u12, u13, u22, u23, u33;  /* g^03 = 0 */
-};
-
 __device__ __forceinline__ Gcon gcon_from(double r, double sth, double cth, double J21, double J22,
                                           double *rho2_out = nullptr, double *irho2_out = nullptr)
 {
@@ -327,13 +251,6 @@ struct PointGeo {
   Met g;
 };
 
-/* r of bl_coord (src/coordinates.c:46-58) */
-template <int MET>
-__device__ __forceinline__ double geo_r(double X1)
-{
-  return (MET == IPG_MET_MINK) ? X1 : exp(X1);
-}
-
 /* flat space in spherical coordinates (src/coordinates.c:180-193) */
 template <int MET>
 __device__ __forceinline__ Met met_flat(double r, double sth)
@@ -373,202 +290,6 @@ __device__ __forceinline__ void point_geo(double X1, double X2, PointGeo *pg)
   sincos(pg->th, &pg->sth, &pg->cth);
   pg->r = r;
   pg->g = met_from(r, pg->sth, pg->cth, pg->J21, pg->J22);
-}
-
-/* --------------------------------------------------------------------- */
-/* Finite-difference connection (src/geometry.c:93-144)                    */
-/* --------------------------------------------------------------------- */
-/* d_d g_{mu nu} for d = 1, 2 (the metric does not depend on X0, X3, so the
- * reference's differences in those directions are exactly zero). */
-struct Conn {
-  Met D1, D2;   /* partial_1 g, partial_2 g */
-  Gcon gu;      /* g^{mu nu} at X */
-  double r;     /* r at X */
-};
-
-__device__ __forceinline__ Met met_diff(const Met &h, const Met &l, double inv)
-{
-  Met d;
-  d.g00 = (h.g00 - l.g00) * inv;
-  d.g01 = (h.g01 - l.g01) * inv;
-  d.g03 = (h.g03 - l.g03) * inv;
-  d.g11 = (h.g11 - l.g11) * inv;
-  d.g12 = (h.g12 - l.g12) * inv;
-  d.g13 = (h.g13 - l.g13) * inv;
-  d.g22 = (h.g22 - l.g22) * inv;
-  d.g33 = (h.g33 - l.g33) * inv;
-  return d;
-}
-
-/* g^{mu nu} of the flat metrics (the reference inverts by LU; diagonal) */
-template <int MET>
-__device__ __forceinline__ Gcon gcon_flat(double r, double sth)
-{
-  Gcon u;
-  u.u00 = -1.;
-  u.u01 = u.u02 = u.u12 = u.u13 = u.u23 = 0.;
-  u.u11 = (MET == IPG_MET_MINK) ? 1. : 1. / (r * r);
-  u.u22 = 1. / (r * r);
-  u.u33 = 1. / (r * r * sth * sth);
-  return u;
-}
-
-template <int MET>
-__device__ void fd_connection_flat(double X1, double X2, Conn *cn)
-{
-  double r = geo_r<MET>(X1), s0, c0;
-  sincos(X2, &s0, &c0);
-  cn->gu = gcon_flat<MET>(r, s0);
-  cn->r = r;
-  {
-    double Xh = X1 + IPG_DEL, Xl = X1 - IPG_DEL;
-    cn->D1 = met_diff(met_flat<MET>(geo_r<MET>(Xh), s0), met_flat<MET>(geo_r<MET>(Xl), s0), 1. / (Xh - Xl));
-  }
-  {
-    double Xh = X2 + IPG_DEL, Xl = X2 - IPG_DEL;
-    cn->D2 = met_diff(met_flat<MET>(r, sin(Xh)), met_flat<MET>(r, sin(Xl)), 1. / (Xh - Xl));
-  }
-}
-
-template <int MET = IPG_MET_FMKS>
-IPG_HEAVY void fd_connection(double X1, double X2, Conn *cn)
-{
-  if constexpr (MET == IPG_MET_MINK || MET == IPG_MET_EMINK) {
-    fd_connection_flat<MET>(X1, X2, cn);
-    return;
-  }
-  const DevGrid &G = c_grid;
-  const double sm = G.mks_smooth;
-  /* center */
-  double r = exp(X1);
-  double E = (MET == IPG_MET_FMKS) ? exp(sm * (G.startx[1] - X1)) : 0.;
-  double S2, C2;
-  sincospi(2. * X2, &S2, &C2);
-  X2P p0;
-  x2_parts_from(X2, S2, C2, &p0);
-  double th0, J21, J22;
-  theta_jac(X2, E, p0, &th0, &J21, &J22);
-  double s0, c0;
-  sincos(th0, &s0, &c0);
-  double rho2c, irho2c;
-  cn->gu = gcon_from(r, s0, c0, J21, J22, &rho2c, &irho2c);
-  cn->r = r;
-
-  /* X1 +- DEL: r and E by exact offsets, theta by its exact difference */
-  {
-    double Xh = X1 + IPG_DEL, Xl = X1 - IPG_DEL;
-    double dh = Xh - X1, dl = Xl - X1; /* exact */
-    double rh = r + r * expm_small(dh), rl = r + r * expm_small(dl);
-    double Eh = E + E * expm_small(-sm * dh), El = E + E * expm_small(-sm * dl);
-    double thh, J21h, J22h, thl, J21l, J22l;
-    theta_jac(X2, Eh, p0, &thh, &J21h, &J22h);
-    theta_jac(X2, El, p0, &thl, &J21l, &J22l);
-    double sd, cd, sh, ch, sl, cl;
-    sincos_small(thh - th0, &sd, &cd);
-    sh = s0 * cd + c0 * sd;
-    ch = c0 * cd - s0 * sd;
-    sincos_small(thl - th0, &sd, &cd);
-    sl = s0 * cd + c0 * sd;
-    cl = c0 * cd - s0 * sd;
-    Met gh = met_from_near(rh, sh, ch, J21h, J22h, rho2c, irho2c);
-    Met gl = met_from_near(rl, sl, cl, J21l, J22l, rho2c, irho2c);
-    cn->D1 = met_diff(gh, gl, 1. / (Xh - Xl));
-  }
-  /* X2 +- DEL */
-  {
-    double Xh = X2 + IPG_DEL, Xl = X2 - IPG_DEL;
-    double dh = Xh - X2, dl = Xl - X2; /* exact */
-    double sd, cd;
-    sincos_small(2. * IPG_PI * dh, &sd, &cd);
-    X2P ph, pl;
-    x2_parts_from(Xh, S2 * cd + C2 * sd, C2 * cd - S2 * sd, &ph);
-    sincos_small(2. * IPG_PI * dl, &sd, &cd);
-    x2_parts_from(Xl, S2 * cd + C2 * sd, C2 * cd - S2 * sd, &pl);
-    double thh, J21h, J22h, thl, J21l, J22l;
-    theta_jac(Xh, E, ph, &thh, &J21h, &J22h);
-    theta_jac(Xl, E, pl, &thl, &J21l, &J22l);
-    double sh, ch, sl, cl;
-    sincos_small(thh - th0, &sd, &cd);
-    sh = s0 * cd + c0 * sd;
-    ch = c0 * cd - s0 * sd;
-    sincos_small(thl - th0, &sd, &cd);
-    sl = s0 * cd + c0 * sd;
-    cl = c0 * cd - s0 * sd;
-    Met gh = met_from_near(r, sh, ch, J21h, J22h, rho2c, irho2c);
-    Met gl = met_from_near(r, sl, cl, J21l, J22l, rho2c, irho2c);
-    cn->D2 = met_diff(gh, gl, 1. / (Xh - Xl));
-  }
-}
-
-/* v = (partial_d g) K */
-__device__ __forceinline__ void dg_dot(const Met &D, const double K[4], double v[4])
-{
-  v[0] = D.g00 * K[0] + D.g01 * K[1] + D.g03 * K[3];
-  v[1] = D.g01 * K[0] + D.g11 * K[1] + D.g12 * K[2] + D.g13 * K[3];
-  v[2] = D.g12 * K[1] + D.g22 * K[2];
-  v[3] = D.g03 * K[0] + D.g13 * K[1] + D.g33 * K[3];
-}
-
-/* Gamma^k_ij K^i K^j (the contraction of push_photon, src/geodesics.c:19-49) */
-__device__ __forceinline__ void geo_accel(const Conn &cn, const double K[4], double acc[4])
-{
-  double v1[4], v2[4], T[4];
-  dg_dot(cn.D1, K, v1);
-  dg_dot(cn.D2, K, v2);
-  double kv1 = K[0] * v1[0] + K[1] * v1[1] + K[2] * v1[2] + K[3] * v1[3];
-  double kv2 = K[0] * v2[0] + K[1] * v2[1] + K[2] * v2[2] + K[3] * v2[3];
-#pragma unroll
-  for (int m = 0; m < 4; m++) T[m] = K[1] * v1[m] + K[2] * v2[m];
-  T[1] -= 0.5 * kv1;
-  T[2] -= 0.5 * kv2;
-  raise(cn.gu, T, acc);
-}
-
-/* A^i_k = Gamma^i_kl K^l (the contraction of push_polar, src/ipolarray.c:253-289) */
-__device__ __forceinline__ void transport_matrix(const Conn &cn, const double K[4], double A[4][4])
-{
-  double v1[4], v2[4], B[4][4];
-  dg_dot(cn.D1, K, v1);
-  dg_dot(cn.D2, K, v2);
-  const Met &D1 = cn.D1, &D2 = cn.D2;
-  /* B[m][k] = 1/2 (K1 d1 g_km + K2 d2 g_km + delta_k1 v1_m + delta_k2 v2_m - delta_m1 v1_k - delta_m2 v2_k) */
-  double d[4][4];
-  d[0][0] = K[1] * D1.g00 + K[2] * D2.g00;
-  d[0][1] = K[1] * D1.g01 + K[2] * D2.g01;
-  d[0][2] = 0.;
-  d[0][3] = K[1] * D1.g03 + K[2] * D2.g03;
-  d[1][1] = K[1] * D1.g11 + K[2] * D2.g11;
-  d[1][2] = K[1] * D1.g12 + K[2] * D2.g12;
-  d[1][3] = K[1] * D1.g13 + K[2] * D2.g13;
-  d[2][2] = K[1] * D1.g22 + K[2] * D2.g22;
-  d[2][3] = 0.;
-  d[3][3] = K[1] * D1.g33 + K[2] * D2.g33;
-  d[1][0] = d[0][1];
-  d[2][0] = d[0][2];
-  d[3][0] = d[0][3];
-  d[2][1] = d[1][2];
-  d[3][1] = d[1][3];
-  d[3][2] = d[2][3];
-#pragma unroll
-  for (int m = 0; m < 4; m++)
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      double b = d[k][m];
-      if (k == 1) b += v1[m];
-      if (k == 2) b += v2[m];
-      if (m == 1) b -= v1[k];
-      if (m == 2) b -= v2[k];
-      B[m][k] = 0.5 * b;
-    }
-  const Gcon &u = cn.gu;
-  double gu[4][4] = {{u.u00, u.u01, u.u02, 0.},
-                     {u.u01, u.u11, u.u12, u.u13},
-                     {u.u02, u.u12, u.u22, u.u23},
-                     {0., u.u13, u.u23, u.u33}};
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int k = 0; k < 4; k++) A[i][k] = gu[i][0] * B[0][k] + gu[i][1] * B[1][k] + gu[i][2] * B[2][k] + gu[i][3] * B[3][k];
 }
 
 /* --------------------------------------------------------------------- */

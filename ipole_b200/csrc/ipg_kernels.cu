@@ -64,26 +64,6 @@ enum { CNT_XDEFER = CNT_N, CNT_BUDGET, CNT_TIMEOUT, CNT_XSTEPS, CNT_NB };
 /* helpers                                                                */
 /* ===================================================================== */
 
-/* src/model_geodesics.c:267-293.  The reference forms three step limits
- * dlx_i = eps c_i / (|K^i| + SS) and returns 1 / sum 1/(|dlx_i| + SS); with
- * a_i = |K^i| + SS and b_i = eps c_i that is
- * dl = eps b1 b2 / (eps (a1 b2 + a2 b1) + a3 b1 b2), one division instead of
- * nine (the + SS of the inner reciprocals matters only for steps near 1e-80,
- * i.e. a ray sitting exactly on the inner or polar boundary). */
-__device__ __forceinline__ double stepsize(const double X[4], const double K[4], double eps)
-{
-  const DevGrid &G = c_grid;
-  const double SS = IPG_SMALL * IPG_SMALL;
-  const double cut = 0.02;
-  double deh = fmin(fabs(X[1] - G.cstartx[1]), 0.1);
-  double dpole = fmin(fabs(X[2] * G.inv_lx2), fabs((G.cstopx[2] - X[2]) * G.inv_lx2));
-  double d2fac = (dpole < cut) ? dpole * (1. / 3.) : fmin(cut * (1. / 3.) + (dpole - cut) * 10., 1.);
-  double a1 = fabs(K[1]) + SS, a2 = fabs(K[2]) + SS, a3 = fabs(K[3]) + SS;
-  double b1 = eps * (10 * deh), b2 = eps * d2fac;
-  double b12 = b1 * b2;
-  return (eps * b12) / (eps * (a1 * b2 + a2 * b1) + a3 * b12);
-}
-
 __device__ __forceinline__ double *step_ptr(double *pool, int chunk, int slot)
 {
   return pool + ((size_t)chunk * IPG_CHUNK_STEPS + slot) * IPG_STEP_DOUBLES;
@@ -168,13 +148,6 @@ __device__ __forceinline__ void load_A_rec(const double *rec, int which, double 
 {
   if (RM < 0 ? c_cam.mixed : RM) load_A_f(reinterpret_cast<const float *>(rec) + (which ? RECM_A2F : RECM_A1F), A);
   else load_A(rec + (which ? REC_A2 : REC_A1), A);
-}
-
-/* Gamma^k_ij K^i K^j = A^k_i K^i */
-__device__ __forceinline__ void accel_from_A(const double A[4][4], const double K[4], double acc[4])
-{
-#pragma unroll
-  for (int k = 0; k < 4; k++) acc[k] = A[k][0] * K[0] + A[k][1] * K[1] + A[k][2] * K[2] + A[k][3] * K[3];
 }
 
 /* Geodesic state of a record.  Xh3 never enters the fast-light computation
@@ -313,9 +286,10 @@ __device__ __forceinline__ void count_turns(const DevCam &C, GeoLane &L)
       if (dX2a * dX2b < 0) L.nturns++;
     } else {
       double ra = geo_r<MET>(L.X1m2), rb = geo_r<MET>(L.X1m1), rc = geo_r<MET>(L.X[1]);
-      double za = ra * cos(bl_theta<MET>(L.X1m2, L.X2m2)), zb = rb * cos(bl_theta<MET>(L.X1m1, L.X2m1));
-      double zc = rc * cos(bl_theta<MET>(L.X[1], L.X[2]));
-      if ((zb - za) * (zc - zb) < 0) L.nturns++;
+      const double za = RN_MUL(ra, cos(bl_theta<MET>(L.X1m2, L.X2m2)));
+      const double zb = RN_MUL(rb, cos(bl_theta<MET>(L.X1m1, L.X2m1)));
+      const double zc = RN_MUL(rc, cos(bl_theta<MET>(L.X[1], L.X[2])));
+      if (RN_SUB(zb, za) * RN_SUB(zc, zb) < 0) L.nturns++;
     }
   }
   L.X1m2 = L.X1m1;
@@ -385,8 +359,7 @@ __global__ void __launch_bounds__(TPB, MINB)
     }
     L.nstep++;
     L.h = -stepsize(L.X, L.K, C.eps);
-#pragma unroll
-    for (int k = 0; k < 4; k++) L.Xh[k] = L.X[k] + 0.5 * L.h * L.K[k];
+    geo_advance(L.X, 0.5 * L.h, L.K, L.Xh);
     Conn c0, c1;
     fd_connection<PlugT<P>::MET>(L.X[1], L.X[2], &c0);
     fd_connection<PlugT<P>::MET>(L.Xh[1], L.Xh[2], &c1);
@@ -398,19 +371,15 @@ __global__ void __launch_bounds__(TPB, MINB)
     } else {
       geo_accel(c0, L.K, acc);
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) L.Kh[k] = L.K[k] - 0.5 * L.h * acc[k];
+    geo_advance(L.K, -0.5 * L.h, acc, L.Kh);
     if (pol) {
       transport_matrix(c1, L.Kh, A);
       accel_from_A(A, L.Kh, acc);
     } else {
       geo_accel(c1, L.Kh, acc);
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      L.K[k] = L.K[k] - L.h * acc[k];
-      L.X[k] = L.X[k] + L.h * L.Kh[k];
-    }
+    geo_advance(L.K, -L.h, acc, L.K);
+    geo_advance(L.X, L.h, L.Kh, L.X);
     double dl = -L.h;
     double dl_cgs = dl * G.L_unit * IPG_HPL / (IPG_ME * IPG_CL * IPG_CL);
     if (track) count_turns<PlugT<P>::MET>(C, L);
@@ -480,19 +449,13 @@ __global__ void __launch_bounds__(TPB, MINB)
       }
       L.nstep++;
       L.h = -stepsize(L.X, L.K, C.eps);
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        L.Kh[k] = L.K[k] - 0.5 * L.h * acc[k];
-        L.Xh[k] = L.X[k] + 0.5 * L.h * L.K[k];
-      }
+      geo_advance(L.K, -0.5 * L.h, acc, L.Kh);
+      geo_advance(L.X, 0.5 * L.h, L.K, L.Xh);
       L.phase = 1;
       continue;
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      L.K[k] = L.K[k] - L.h * acc[k];
-      L.X[k] = L.X[k] + L.h * L.Kh[k];
-    }
+    geo_advance(L.K, -L.h, acc, L.K);
+    geo_advance(L.X, L.h, L.Kh, L.X);
     L.phase = 0;
     double dl = -L.h;
     double dl_cgs = dl * G.L_unit * IPG_HPL / (IPG_ME * IPG_CL * IPG_CL);
@@ -572,18 +535,12 @@ __global__ void __launch_bounds__(128, IPG_GEO_MINB)
     if (phase == 0) {
       nstep++;
       h = -stepsize(X, K, eps);
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        Kh[k] = K[k] - 0.5 * h * acc[k];
-        Xh[k] = X[k] + 0.5 * h * K[k];
-      }
+      geo_advance(K, -0.5 * h, acc, Kh);
+      geo_advance(X, 0.5 * h, K, Xh);
       phase = 1;
     } else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        K[k] = K[k] - h * acc[k];
-        X[k] = X[k] + h * Kh[k];
-      }
+      geo_advance(K, -h, acc, K);
+      geo_advance(X, h, Kh, X);
       phase = 0;
     }
   }

@@ -55,13 +55,13 @@ __device__ __forceinline__ double bl_theta(double X1, double X2)
 {
   if constexpr (MET == IPG_MET_MINK || MET == IPG_MET_EMINK) return X2;
   const DevGrid &G = c_grid;
-  double E = (MET == IPG_MET_FMKS) ? exp(G.mks_smooth * (G.startx[1] - X1)) : 0.;
+  double E = (MET == IPG_MET_FMKS) ? exp(RN_MUL(G.mks_smooth, RN_SUB(G.startx[1], X1))) : 0.;
   double S2, C2;
   sincospi(2. * X2, &S2, &C2);
   X2P p;
   x2_parts_from(X2, S2, C2, &p);
   double th, j1, j2;
-  theta_jac(X2, E, p, &th, &j1, &j2);
+  conn_theta(X2, E, p, &th, &j1, &j2);
   return th;
 }
 

@@ -1,0 +1,141 @@
+/* ipg_connection.cuh compiled for the host (tests/test_connection.py): prints
+ * the bits that its functions give along geodesics, and compares the lanes'
+ * shares of k_geodesic_coop, evaluated one after another, with the one-lane
+ * form of k_geodesic. */
+#include <math.h>
+#include <stdint.h>
+#include <stdio.h>
+#include <string.h>
+
+#define __device__
+#define __forceinline__ inline
+#define IPG_HEAVY static
+#define IPG_DEL 1.e-7
+#define IPG_SMALL (1.e-40)
+#define IPG_PI 3.14159265358979323846
+enum { IPG_MET_FMKS, IPG_MET_MKS, IPG_MET_MINK, IPG_MET_EMINK };
+struct DevGrid {
+  int alpha_int;
+  double startx[4], cstartx[4], cstopx[4];
+  double a, hslope, poly_xt, poly_alpha, mks_smooth, poly_norm, inv_xt, inv_ap1, j22c, inv_lx2;
+};
+static DevGrid c_grid;
+/* a rounding that nothing is fused across */
+static inline double pin(double x)
+{
+  asm volatile("" : "+x"(x));
+  return x;
+}
+static inline double __dmul_rn(double a, double b) { return pin(pin(a) * pin(b)); }
+static inline double __dadd_rn(double a, double b) { return pin(pin(a) + pin(b)); }
+static inline double __dsub_rn(double a, double b) { return pin(pin(a) - pin(b)); }
+static inline double __fma_rn(double a, double b, double c) { return pin(fma(a, b, c)); }
+static inline void sincospi(double x, double *s, double *c)
+{
+  const double t = pin(IPG_PI * x);
+  *s = sin(t);
+  *c = cos(t);
+}
+#include "ipg_connection.cuh"
+
+static unsigned long long hash = 1469598103934665603ULL;
+static void put(const double *v, int n)
+{
+  for (int i = 0; i < n; i++) {
+    uint64_t u;
+    memcpy(&u, v + i, 8);
+    hash = (hash ^ u) * 1099511628211ULL;
+  }
+}
+static unsigned long long seed = 12345;
+static double rnd(double lo, double hi)
+{
+  seed = seed * 6364136223846793005ULL + 1442695040888963407ULL;
+  return pin(lo + pin((hi - lo) * ((double)(seed >> 11) / 9007199254740992.)));
+}
+
+/* the metric of lane o, as gc_connection selects it */
+static void lane_metric(double X1, double X2, int o, double g[8], Conn *p, double *dx)
+{
+  ConnCentre c;
+  const double sm = c_grid.mks_smooth;
+  conn_centre<true>(exp(X1), exp(__dmul_rn(sm, __dsub_rn(c_grid.startx[1], X1))), X2, &c, &p->gu);
+  const double Xc = o < 2 ? X1 : X2, Xh = __dadd_rn(Xc, IPG_DEL), Xl = __dsub_rn(Xc, IPG_DEL);
+  const double Xo = (o & 1) ? Xl : Xh, d = __dsub_rn(Xo, Xc), d1 = o < 2 ? d : 0., d2 = o < 2 ? 0. : d;
+  double sd, cd, S, C;
+  sincos_small(__dmul_rn(2. * IPG_PI, d2), &sd, &cd);
+  rotate(c.p.S2, c.p.C2, sd, cd, &S, &C);
+  X2P po;
+  const double X2o = o < 2 ? X2 : Xo;
+  x2_parts_from<true>(X2o, S, C, &po);
+  ConnOffset off;
+  conn_offset(c, __fma_rn(c.E, expm_small(__dmul_rn(-sm, d1)), c.E), X2o, po, &off);
+  conn_near(c, __fma_rn(c.r, expm_small(d1), c.r), off, o >= 2, g);
+  *dx = __dsub_rn(Xh, Xl);
+}
+
+int main()
+{
+  long lanes_differ = 0;
+  for (int alpha = 0; alpha < 3; alpha++) {
+    DevGrid &G = c_grid;
+    G.poly_alpha = alpha == 0 ? 14. : alpha == 1 ? 8. : 11.5;
+    G.alpha_int = alpha == 2 ? -1 : (int)G.poly_alpha - 1;
+    G.a = 0.9375;
+    G.hslope = 0.3;
+    G.mks_smooth = 0.5;
+    G.poly_xt = 0.82;
+    G.poly_norm = 0.757817;
+    G.inv_xt = 1. / G.poly_xt;
+    G.inv_ap1 = 1. / (G.poly_alpha + 1.);
+    G.j22c = 2. * G.poly_alpha * G.poly_norm / ((1. + G.poly_alpha) * G.poly_xt);
+    G.startx[1] = G.cstartx[1] = 0.2;
+    G.cstopx[1] = 4.;
+    G.cstopx[2] = 1.;
+    G.inv_lx2 = 1.;
+    for (int ray = 0; ray < 300; ray++) {
+      double X[4] = {0., rnd(0.4, 6.4), rnd(0.02, 0.98), rnd(0., 1.)};
+      if (alpha == 2) X[2] = rnd(0.55, 0.98); /* a power of a positive base only */
+      double K[4] = {rnd(1., 2.), rnd(-0.1, 0.1), rnd(-0.01, 0.01), rnd(-0.1, 0.1)};
+      for (int n = 0; n < 40; n++) {
+        Conn cn;
+        double A[4][4], acc[4], au[4], Xh[4], Kh[4];
+        fd_connection(X[1], X[2], &cn);
+        for (int o = 0; o < 4; o++) {
+          Conn p;
+          double g[2][8], dx;
+          lane_metric(X[1], X[2], o & 2, g[0], &p, &dx);
+          lane_metric(X[1], X[2], (o & 2) | 1, g[1], &p, &dx);
+          lanes_differ += memcmp(&p.gu, &cn.gu, sizeof(p.gu)) != 0;
+          for (int k = 0; k < 8; k++) {
+            const double d = conn_diff(g[0][k], g[1][k], 1. / dx), e = (o & 2) ? cn.D2[k] : cn.D1[k];
+            lanes_differ += memcmp(&d, &e, 8) != 0;
+          }
+        }
+        transport_matrix(cn, K, A);
+        accel_from_A(A, K, acc);
+        geo_accel(cn, K, au);
+        put(cn.D1, 8);
+        put(cn.D2, 8);
+        put(&cn.gu.u00, 9);
+        put(A[0], 16);
+        put(acc, 4);
+        put(au, 4);
+        const double h = -stepsize(X, K, 0.01);
+        put(&h, 1);
+        geo_advance(X, 0.5 * h, K, Xh);
+        geo_advance(K, -0.5 * h, acc, Kh);
+        fd_connection(Xh[1], Xh[2], &cn);
+        transport_matrix(cn, Kh, A);
+        accel_from_A(A, Kh, acc);
+        geo_advance(K, -h, acc, K);
+        geo_advance(X, h, Kh, X);
+        put(X, 4);
+        put(K, 4);
+        if (!(X[1] > 0.3) || !(X[1] < 8.) || !(X[2] > (alpha == 2 ? 0.51 : 0.001)) || !(X[2] < 0.999)) break;
+      }
+    }
+  }
+  printf("%016llx %ld\n", hash, lanes_differ);
+  return 0;
+}

@@ -35,6 +35,9 @@ int ipg__fits32(const ipg_ctx *ctx);
 /* self-check of the adjoint's reverse-mode transfer step against forward
  * dual numbers on n seeded cases; *max_err the largest relative difference */
 int ipg__check_step_vjp(int device, int n, unsigned long long seed, double max_err[4], double worst[96]);
+/* self-check of the eight-lane geodesic's reciprocal against the division, on
+ * n seeded arguments of three kinds; bad[k] = those that differ */
+int ipg__check_recip(int device, int n, unsigned long long seed, double width, unsigned long long bad[3]);
 /* per-context storage of the batch driver (ipg_refine.cu); ipg_destroy
  * releases it with ipg__batch_arena_release */
 void **ipg__batch_arena_slot(ipg_ctx *ctx);

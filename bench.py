@@ -58,12 +58,18 @@ CPU_SAMPLE = 64  # reference / oracle sample image size (pixels per side)
 # rest.
 REF_FLOPS = {"geodesic_per_step": 24172.6, "push_per_step": 30454.0, "coeffs_per_radiating_step": 8942.3,
              "transfer_per_radiating_step": 4751.9}
-# What the kernels execute per ray-step, from the ncu capture of a 200x200
+# What the kernels execute per ray-step, from an ncu capture of a 200x200
 # image of the 128x64x64 dump: FP64 flops (2 per DFMA, 1 per DADD/DMUL) and
-# DRAM bytes read + written (k_coeffs works per step record; the walk is
-# k_walk with four lanes per ray).
-EXEC_FLOPS_PER_STEP = {"geodesic": 1831, "coeffs": 1535, "transfer": 913}
-DRAM_BYTES_PER_STEP = {"geodesic": 377, "coeffs": 411, "transfer": 542}
+# DRAM bytes read + written, of the forms that every class of the 400x400
+# image launches: the geodesic with one lane per ray and the walk with four
+# (k_walk<4>; with IPG_XFER_STAGE=0 k_transfer).  Smaller images launch forms
+# with more lanes per ray, which execute more (eight-lane geodesic 5482,
+# k_walk<8> 2224).
+EXEC_FLOPS_PER_STEP = {"geodesic": 1830, "coeffs": 1559, "transfer": 1226}
+DRAM_BYTES_PER_STEP = {"geodesic": 377, "coeffs": 424, "transfer": 541}
+ONE_LANE_WALK = os.environ.get("IPG_XFER_STAGE", "").startswith("0")
+if ONE_LANE_WALK:
+    EXEC_FLOPS_PER_STEP["transfer"], DRAM_BYTES_PER_STEP["transfer"] = 913, 537
 
 
 def data_dir():
@@ -408,15 +414,11 @@ def run_ours(args):
     alg_total = sum(alg.values())
     exec_total = sum(EXEC_FLOPS_PER_STEP.values()) * steps
     traffic = DRAM_BYTES_PER_STEP[dom] * (steps / args.steps)
-    # the transfer walk has several lanes per ray (k_walk) unless
-    # IPG_XFER_STAGE=0 selects one lane per ray
-    walk = "k_transfer" if os.environ.get("IPG_XFER_STAGE", "").startswith("0") else "k_walk"
-    kname = walk if dom == "transfer" else f"k_{dom}"
+    kname = ("k_transfer" if ONE_LANE_WALK else "k_walk") if dom == "transfer" else f"k_{dom}"
     roofline = {"bound": "fp64", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                 "traffic_note": "DRAM bytes per image (all class launches of the kernel): ncu bytes per ray-step "
-                                "of a small case of the 128x64x64 dump (the walk: its bulk-copy form on an "
-                                "unsplit 256x256 wave) times this image's ray-steps",
+                                "of a 200x200 image of the 128x64x64 dump times this image's ray-steps",
                 "frac_pipeline": alg_total / (ms / 1e3) / 1e12 / peak,
                 "frac_pipeline_executed": exec_total / (ms / 1e3) / 1e12 / peak,
                 "alg_flops_per_ray_step": alg_total / max(steps, 1),
@@ -424,7 +426,8 @@ def run_ours(args):
                 "alg_note": "algorithmic = the reference algorithm's FP64 operations counted with a counting "
                             "number type (transcendentals 20 flops); the kernels execute ~15x fewer (analytic "
                             "connection and metric instead of finite differences of gcov with LU inversions), "
-                            "so the algorithmic fractions can exceed 1; *_executed uses ncu's executed FP64 flops",
+                            "so the algorithmic fractions can exceed 1; *_executed uses ncu's executed FP64 flops "
+                            "of the forms that a 400x400 image launches",
                 "kernels": kern, "hbm_GBps_of_dominant": traffic * args.steps / (span[dom] / 1e3) / 1e9,
                 "peak_source": "measured in this run: FP64 FMA loop (ipg_measure_fp64_peak); MEASURED_PEAKS.json "
                                "has no FP64 figure",

@@ -1392,12 +1392,12 @@ struct ipg_ctx {
   ipg_stats stats;
   void *refine; /* buffers of the on-device image driver (ipg_refine.cu) */
   double *d_trace_extra; /* rho, u, beta per cell for the trace output (ipg_upload_trace_fields) */
-  /* the adjoint's scratch, kept between calls (grow-only): dL/dout per
-   * pixel, the cells' gradients, the walk's links */
   double *d_upload; /* upload_fields' scratch */
   double *d_coef;   /* ipg_thermal_coefficients' workspace: coef_cap points, in use while coef_busy */
   size_t coef_cap;
   int coef_busy;
+  /* the adjoint's scratch, kept between calls (grow-only): dL/dout per
+   * pixel, the cells' gradients, the walk's links */
   double *d_adj_dl, *d_adj_g;
   int *d_adj_next, *d_adj_first;
   size_t adj_dl_cap, adj_g_cap, adj_next_cap, adj_first_cap;
@@ -1455,9 +1455,9 @@ extern "C" int ipg_create(ipg_ctx **out, int device, size_t pool_bytes)
   for (int i = 0; e == cudaSuccess && i < 5; i++) e = cudaEventCreate(&ctx->ev[i]);
   /* the length classes' streams share the highest priority.  Ranking them
    * (longest class first) measured 199-205 ms per 400x400 image against
-   * 190-198 ms for equal ranks: once the shorter classes' coefficient passes
-   * wait for the longest class's geodesics, the end of the image is the
-   * shortest class's chain, which a lower rank delays. */
+   * 190-198 ms for equal ranks when the shorter classes' coefficient passes
+   * still waited for the longest class's geodesics; not measured since they
+   * do not. */
   int prio_lo = 0, prio_hi = 0;
   if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
   for (int b = 0; e == cudaSuccess && b < NB_MAX; b++) {
@@ -1809,8 +1809,9 @@ static void wait_started(ipg_ctx *ctx, int n)
 
 /* One batch of a wave: a slice of a ray list, a slice of the trajectory pool
  * and its own counters, run as geodesic -> coefficients -> transfer on one
- * stream.  wide = 1 launches the two sequential kernels in 256-thread blocks,
- * whose registers fill an SM: no block of another kernel fits beside them. */
+ * stream.  wide = 1 (the longest class) launches k_geodesic, and k_transfer, in
+ * 256-thread blocks, whose registers fill an SM; k_geodesic_coop's wide blocks
+ * go by split instead (IPG_COOP_WIDE), and k_walk's are one warp always. */
 struct Batch {
   const int32_t *list;
   size_t run;
@@ -1891,8 +1892,8 @@ static int launch_geo_coop(ipg_ctx *ctx, int unpol, int mixed, int wide, const i
  * wave sorted longest first, the head of the list takes it on a stream of its
  * own, on SMs of its own: a wave ends on its longest rays, whose step takes
  * 1.7 us there and 3.1 us or more with a lane per ray.  The head is an eighth
- * of the rays, at most eight per SM (25 blocks of 48 rays: a sixth of the
- * SMs): what follows is then under three times the mean length, which a lane
+ * of the rays, at most eight per SM (37 blocks, a quarter of the SMs, of 32
+ * rays each): what follows is then under three times the mean length, which a lane
  * per ray walks within the time of the whole wave.  Both take their records
  * from the same pool, by the same counters; each has its own queue. */
 template <class CS>
@@ -2028,10 +2029,11 @@ static int launch_transfer(ipg_ctx *ctx, const Batch &b, ipg_pixel_out *d_out)
 template <int P>
 static int launch_batch_t(ipg_ctx *ctx, const Batch &b, const int32_t *d_ij, ipg_pixel_out *d_out)
 {
-  /* Every class launches the same compiled geodesic and transfer kernels
-   * (SM-filling blocks for the longest class, 128-thread blocks, two per SM,
-   * for the others): classes that run side by side then share their
-   * instructions instead of competing for instruction-cache space. */
+  /* Classes that take one lane per ray launch the same compiled geodesic
+   * (256-thread blocks for the longest class, 128-thread blocks, two per SM,
+   * for the others): side by side they share its instructions instead of
+   * competing for instruction-cache space.  Classes of few rays take
+   * k_geodesic_coop, and each class's walk the lanes that its size gives. */
   const int threads = 128;
   const int gthreads = b.wide ? 256 : threads;
   CK(cudaEventRecord(b.ev[0], b.stream));

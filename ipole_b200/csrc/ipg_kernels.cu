@@ -1339,15 +1339,22 @@ static void devgrid_derived(DevGrid *d)
 
 /* Length classes of a split wave: rays predicted at least facs[c] times the
  * mean length go to class c (the first class runs wide), the rest to the
- * last class.  A wave of more than two resident grids of k_geodesic (512 rays
- * per SM) is bound by the throughput of its last class, geodesics,
+ * last class.  A polarized wave of more than two resident grids of k_geodesic
+ * (512 rays per SM) is bound by the throughput of its last class, geodesics,
  * coefficients, walk; its middle class at 2 to 4 times the mean ended later
  * than that, so there the longest class takes rays from 2.5 times the mean
- * and the middle one those from 1.5.  ms per image, 4 and 2 / 2.5 and 1.5:
- * 400x400 161 / 142 (mixed tier 133 / 128), 280x280 91 / 74, 96 / 72 (128x64x64
- * dump, mixed), 360x360 98 / 96; but 230x230 (52 900 rays) 56 / 59, 128x128 36 /
- * 37, and unpolarized images, which end on their longest rays, 340x340 70 /
- * 71. */
+ * and the middle one those from 1.5: but not where the rays from 2.5 times the
+ * mean are 22 to 34 per SM (class_facs).  Up to 22 they take eight lanes each
+ * (k_geodesic_coop) on under half the SMs, above 34 one lane each on a sixth;
+ * between, eight lanes each hold half to two thirds of the SMs while the rest
+ * waits, and just above geo_coop's 32 one lane each ends late.  Image time with
+ * 2.5 / 1.5 over that with 4 / 2, mean of ten cameras and dumps (mixed tier in
+ * brackets): 276x276 (18 per SM) 0.83 (0.82), 290 (20) 0.84 (0.82), 300 (21)
+ * 0.98 (0.96); 310 (23) 0.96 (0.98, cameras up to 1.13), 320 (24) 1.04 (1.06),
+ * 345 (28) 1.04 (1.13), 360 (30) 0.98 (0.95, up to 1.07), 370 (32) 1.04 (1.04,
+ * up to 1.26); 385 (35) 0.97 (0.99), 400 (37) 0.97 (0.95).  Below 512 rays per
+ * SM 4 and 2 stay: 230x230 56 against 59 ms, 128x128 36 against 37; and for
+ * unpolarized images, which end on their longest rays, 340x340 70 against 71. */
 static const double k_class_facs[] = {4., 2.}, k_class_facs_large[] = {2.5, 1.5};
 #define NB_MAX ((int)(sizeof(k_class_facs) / sizeof(k_class_facs[0])) + 1)
 static_assert(sizeof(k_class_facs) == sizeof(k_class_facs_large), "the same number of classes");
@@ -2140,6 +2147,16 @@ static void launch_count_t(ipg_ctx *ctx, int threads, const int32_t *d_ij, const
 }
 #define SPLIT_MIN_RAYS 4096
 
+/* the thresholds for a wave of `run` rays with this histogram of lengths */
+static const double *class_facs(const ipg_ctx *ctx, int unpol, size_t run, const int *hist, double mean)
+{
+  const size_t sm = (size_t)ctx->n_sm;
+  if (unpol || run <= sm * 512) return k_class_facs;
+  size_t c = 0;
+  for (int b = (int)(k_class_facs_large[0] * mean) + 1; b < LEN_BUCKETS; b++) c += (size_t)hist[b];
+  return c > sm * 22 && c <= sm * 34 ? k_class_facs : k_class_facs_large;
+}
+
 static int plan_split(ipg_ctx *ctx, const int32_t *d_ij, const int32_t *list, size_t run, const ipg_camera *cam,
                       int *nb, size_t sizes[NB_MAX], double shares[NB_MAX], int wide[NB_MAX])
 {
@@ -2173,8 +2190,7 @@ static int plan_split(ipg_ctx *ctx, const int32_t *d_ij, const int32_t *list, si
    * after all are deferred to the next wave like any other */
   if (total * PRED_EPS_SCALE > (double)ctx->n_chunks * IPG_CHUNK_STEPS) return IPG_OK;
   double mean = total / (double)run;
-  const double *facs =
-      !cam->only_unpolarized && run > (size_t)ctx->n_sm * 512 ? k_class_facs_large : k_class_facs;
+  const double *facs = class_facs(ctx, cam->only_unpolarized, run, hist.data(), mean);
   int hi = LEN_BUCKETS; /* classes are bucket ranges [thr, hi) */
   size_t used = 0;
   int n = 0;

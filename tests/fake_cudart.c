@@ -30,6 +30,7 @@ static char fail_name[64];
 static cudaError_t last;
 static float elapsed_ms = 1.f;
 static float (*elapsed_cb)(void);
+static void (*launch_cb)(const char *, void **);
 
 /* ---- the tests' side ---- */
 static void sync_all(void)
@@ -63,6 +64,8 @@ int fake_inflight(cudaStream_t but)
 }
 const char *fake_log(void) { return log_; } /* the launched kernels' names, a line each */
 void fake_elapsed(float (*cb)(void)) { elapsed_cb = cb; }
+/* stands in for the kernels: called with each launch's kernel name and arguments */
+void fake_on_launch(void (*cb)(const char *, void **)) { launch_cb = cb; }
 
 static void enqueue(cudaStream_t s) { (s ? s : streams)->pending++; }
 static void finish(cudaStream_t s)
@@ -120,6 +123,8 @@ cudaError_t cudaLaunchKernel(const void *fn, dim3 g, dim3 b, void **args, size_t
   FAIL();
   n_launch++;
   enqueue(st);
+  for (int i = 0; launch_cb && i < n_kern; i++)
+    if (kern[i].fn == fn) launch_cb(kern[i].name, args);
   for (int i = 0; i < n_kern; i++)
     if (kern[i].fn == fn && strlen(log_) + strlen(kern[i].name) + 2 < sizeof(log_)) {
       strcat(log_, kern[i].name);

@@ -59,3 +59,30 @@ for sizes in ([70000], [100, 100, 70000], [70000, 70000, 70000]):
         c.close()
 assert len(seen) == 1, seen
 """)
+
+
+@pytest.mark.parametrize("side,large", [(270, False), (290, True), (300, True), (320, False), (345, False), (370, False),
+                                        (400, True)])
+def test_longest_class_of_large_images(lib, side, large):
+    """3.45% of the rays 3 times the mean long or longer and 0.4% 5 times, as in
+    images of the synthetic dumps: the longest class starts at 2.5 times the
+    mean where that holds at most 22 rays per SM or more than 34 (148 SMs),
+    else, and in smaller images, at 4 times"""
+    fake_cuda.run(lib, f"""
+n = {side} ** 2
+geo = []
+def kernel(name, args):
+    at = lambda k, t: C.cast(args[k], C.POINTER(t))[0]
+    if b"k_len_hist" in name:
+        hist = C.cast(at(3, C.c_void_p), C.POINTER(C.c_int))
+        hist[40], hist[24], hist[7] = int(.004 * n), int(.0305 * n), n - int(.004 * n) - int(.0305 * n)
+    elif b"k_geodesic" in name and b"count" not in name:
+        geo.append(at(2, C.c_int))
+cb = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p))(kernel)
+L.fake_on_launch(cb)
+c = ip.Context(0, 8 << 30)
+g = grid(2, 2, 2)
+c.upload_arrays(g, fields(g))
+assert code(c.trace, camera(nx={side}, ny={side}), np.zeros((n, 2), np.int32)) == 0
+assert sum(geo) == n and geo[0] == int(.004 * n) + ({large} and int(.0305 * n)), geo
+""")

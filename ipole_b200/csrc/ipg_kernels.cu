@@ -449,8 +449,12 @@ __global__ void __launch_bounds__(TPB, MINB)
       }
       L.nstep++;
       L.h = -stepsize(L.X, L.K, C.eps);
-      geo_advance(L.K, -0.5 * L.h, acc, L.Kh);
-      geo_advance(L.X, 0.5 * L.h, L.K, L.Xh);
+      const double hh = 0.5 * L.h;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        L.Kh[k] = RN_FMA(-hh, acc[k], L.K[k]);
+        L.Xh[k] = RN_FMA(hh, L.K[k], L.X[k]);
+      }
       L.phase = 1;
       continue;
     }

@@ -55,11 +55,12 @@ static double rnd(double lo, double hi)
 }
 
 /* the metric of lane o, as gc_connection selects it */
+template <bool HALF>
 static void lane_metric(double X1, double X2, int o, double g[8], Conn *p, double *dx)
 {
   ConnCentre c;
   const double sm = c_grid.mks_smooth;
-  conn_centre<true>(exp(X1), exp(__dmul_rn(sm, __dsub_rn(c_grid.startx[1], X1))), X2, &c, &p->gu);
+  conn_centre<true, HALF>(exp(X1), exp(__dmul_rn(sm, __dsub_rn(c_grid.startx[1], X1))), X2, &c, &p->gu);
   const double Xc = o < 2 ? X1 : X2, Xh = __dadd_rn(Xc, IPG_DEL), Xl = __dsub_rn(Xc, IPG_DEL);
   const double Xo = (o & 1) ? Xl : Xh, d = __dsub_rn(Xo, Xc), d1 = o < 2 ? d : 0., d2 = o < 2 ? 0. : d;
   double sd, cd, S, C;
@@ -103,14 +104,21 @@ int main()
         fd_connection(X[1], X[2], &cn);
         for (int o = 0; o < 4; o++) {
           Conn p;
-          double g[2][8], dx;
-          lane_metric(X[1], X[2], o & 2, g[0], &p, &dx);
-          lane_metric(X[1], X[2], (o & 2) | 1, g[1], &p, &dx);
+          double g[2][8], dx, B[4][4], Ao[4];
+          lane_metric<false>(X[1], X[2], o & 2, g[0], &p, &dx);
+          lane_metric<false>(X[1], X[2], (o & 2) | 1, g[1], &p, &dx);
           lanes_differ += memcmp(&p.gu, &cn.gu, sizeof(p.gu)) != 0;
           for (int k = 0; k < 8; k++) {
             const double d = conn_diff(g[0][k], g[1][k], 1. / dx), e = (o & 2) ? cn.D2[k] : cn.D1[k];
             lanes_differ += memcmp(&d, &e, 8) != 0;
           }
+          /* the lane's row of A, from half of g^{mu nu} */
+          p = cn;
+          lane_metric<true>(X[1], X[2], o, g[0], &p, &dx);
+          transport_b(p, K, B);
+          transport_row(p.gu, B, o, Ao);
+          transport_matrix(cn, K, A);
+          lanes_differ += memcmp(Ao, A[o], sizeof(Ao)) != 0;
         }
         transport_matrix(cn, K, A);
         accel_from_A(A, K, acc);
